@@ -781,6 +781,7 @@ template <typename R, bool ONE = false> struct EngineIo
   __device__ __forceinline__ void put(int c, R v) const { ipw<R>(M, c, q, v); }
   __device__ __forceinline__ void slot(const R4 &v) const { reinterpret_cast<R4 *>(M.slot)[M.slot_pos[q]] = v; }
   __device__ __forceinline__ const float *ip32() const { return reinterpret_cast<const float *>(M.ip); }
+  __device__ __forceinline__ int ip32_index() const { return q; }
   __device__ __forceinline__ void first_node(unsigned amask, int base, const double4 &X, const double4 &U,
                                              double4 &X0, double4 &U0) const
   {
@@ -898,12 +899,14 @@ __device__ __forceinline__ void kinematics(unsigned amask, int g, int base, cons
 // radial return, final rotation, density, and the element's nodal forces,
 // summed over its points through shared memory and stored in node order.
 // `row` is this lane's shared-memory row, `grp` the row of the element's first lane.
+// C: the instance's control values (the global block, or a block's own copy of
+// it); G: the global control block, which takes errors and counts.
 // The element-pass modes run the same update split in two (element_front /
 // element_back below); this single body is what the plain variants use (the
 // split costs the plain variants about 10 % in spilled registers).
 template <typename R, int NPE, class Src, class Io>
-__device__ __forceinline__ void element_update(const Io &io, Ctl *C, int q, int e, int g, int base, unsigned amask,
-                                               int node, const Src &old, R *row, R *grp)
+__device__ __forceinline__ void element_update(const Io &io, const Ctl *C, Ctl *G, int q, int e, int g, int base,
+                                               unsigned amask, int node, const Src &old, R *row, R *grp)
 {
   constexpr int DIM = ElemShape<NPE>::DIM;
   const bool AXI = ElemShape<NPE>::AXI && !(C->plane);
@@ -921,7 +924,7 @@ __device__ __forceinline__ void element_update(const Io &io, Ctl *C, int q, int 
     polar_lnU<R>(H, dE, Rot);
   }
   if (detJ < R(0))
-    raise_status(C, DNL_ERR_NEG_JACOBIAN, e);
+    raise_status(G, DNL_ERR_NEG_JACOBIAN, e);
   R WxdJ = detJ; // Gauss weight 1
   if (AXI)
     WxdJ *= R(6.28318530717958647692) * radius;
@@ -966,11 +969,11 @@ __device__ __forceinline__ void element_update(const Io &io, Ctl *C, int q, int 
     {
       if constexpr (sizeof(R) == 4)
       {
-        atomicAdd(&C->resolves, 1);
-        const Resolved r = resolve_fp64(io.ip32(), q, io.matp(e), dE[0], dE[1], dE[2], dE[3], dE[4], dE[5], dt,
+        atomicAdd(&G->resolves, 1);
+        const Resolved r = resolve_fp64(io.ip32(), io.ip32_index(), io.matp(e), dE[0], dE[1], dE[2], dE[3], dE[4], dE[5], dt,
                                         st.pressure);
         if (!r.ok)
-          raise_status(C, DNL_ERR_NEWTON, q);
+          raise_status(G, DNL_ERR_NEWTON, q);
 #pragma unroll
         for (int c = 0; c < 6; c++)
           st.s[c] = r.s[c];
@@ -985,7 +988,7 @@ __device__ __forceinline__ void element_update(const Io &io, Ctl *C, int q, int 
         st.einel = r.einel;
       }
       else
-        raise_status(C, DNL_ERR_NEWTON, q);
+        raise_status(G, DNL_ERR_NEWTON, q);
     }
   }
 
@@ -1434,7 +1437,7 @@ __global__ void __launch_bounds__(PTS, MINB) k_element(DevModel M, int nTiles)
     return;
   GlobalState<R> old{M, q};
   EngineIo<R, ONE> io{M, q, C->f0};
-  element_update<R, NPE>(io, C, q, e, g, base, amask, M.conn[q], old, sh + threadIdx.x * ROW,
+  element_update<R, NPE>(io, C, C, q, e, g, base, amask, M.conn[q], old, sh + threadIdx.x * ROW,
                          sh + (threadIdx.x - g) * ROW);
 }
 
@@ -1566,7 +1569,7 @@ __global__ void __launch_bounds__(TILE, MINB) k_element_tma(DevModel M, int nTil
     {
       SharedTile<R> old{state[b], t};
       EngineIo<R, ONE> io{M, q, C->f0};
-      element_update<R, NPE>(io, C, q, e, g, base, amask, conn[b][t], old, rows + t * ROW, rows + (t - g) * ROW);
+      element_update<R, NPE>(io, C, C, q, e, g, base, amask, conn[b][t], old, rows + t * ROW, rows + (t - g) * ROW);
     }
     __syncthreads(); // the buffer is refilled two tiles later
   }
@@ -1633,6 +1636,7 @@ template <typename R, bool ONE = false> struct StagedIo
   __device__ __forceinline__ void put(int c, R v) const { ipw<R>(M, c, q, v); }
   __device__ __forceinline__ void slot(const R4 &v) const { reinterpret_cast<R4 *>(M.slot)[spos] = v; }
   __device__ __forceinline__ const float *ip32() const { return reinterpret_cast<const float *>(M.ip); }
+  __device__ __forceinline__ int ip32_index() const { return q; }
   // the element's first node is staged g entries before this lane's
   __device__ __forceinline__ void first_node(unsigned, int, const double4 &, const double4 &, double4 &X0,
                                              double4 &U0) const
@@ -1795,7 +1799,7 @@ __global__ void __launch_bounds__(TILE, MINB) k_element_stage(DevModel M, int nT
       SharedTile<R> old{state(b), t};
       StagedIo<R, ONE> io{M, q, {nxy(b, 0) + t, nz(b, 0) + t}, {nxy(b, 1) + t, nz(b, 1) + t}, spos(b)[t],
                      M.mat + emat(b)[t / NPE], g};
-      element_update<R, NPE>(io, C, q, e, g, base, amask, 0, old, rows + t * ROW, rows + (t - g) * ROW);
+      element_update<R, NPE>(io, C, C, q, e, g, base, amask, 0, old, rows + t * ROW, rows + (t - g) * ROW);
     }
     __syncthreads(); // the buffers of this tile are refilled from the next iteration on
     cur = next;
@@ -2073,16 +2077,8 @@ __global__ void __launch_bounds__(NODAL_THREADS) k_nodal_batch(DevModel M)
 
 // Predictor boundary conditions on field0 of the imposed-speed nodes before the
 // element pass (the element pass reads field0->u, Element.C:1114).
-__global__ void k_bc_prep(DevModel M)
+__device__ __forceinline__ void bc_prep_node(const DevModel &M, int i, const Ctl *C)
 {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= M.nSpeed)
-    return;
-  const int i = M.speed_nodes[k];
-  const int inst = (M.nInst > 1) ? find_segment(M.inst_node_begin, M.nInst, i) : 0;
-  const Ctl *C = M.ctl + inst;
-  if (!C->active)
-    return;
   const double dt = C->dt_eff, t = C->t;
   const int f0 = C->f0;
   const unsigned code = M.bc[i];
@@ -2110,6 +2106,18 @@ __global__ void k_bc_prep(DevModel M)
   M.u[f0][i] = u0;
   M.v[f0][i] = v0;
   M.a[f0][i] = a0;
+}
+
+__global__ void k_bc_prep(DevModel M)
+{
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= M.nSpeed)
+    return;
+  const int i = M.speed_nodes[k];
+  const int inst = (M.nInst > 1) ? find_segment(M.inst_node_begin, M.nInst, i) : 0;
+  const Ctl *C = M.ctl + inst;
+  if (C->active)
+    bc_prep_node(M, i, C);
 }
 
 // Sum the element slots of every node (lumped mass at the start, or the
@@ -2838,10 +2846,8 @@ __global__ void k_slot_pos(DevModel M, BuildRaw R, int W)
 // Nodal vector `field` (DNL_NODE_*) of node i, on the parity of the two-buffer
 // fields of the node's instance (field0 = the current values; the _PREV
 // fields the other buffer, the values before the last increment).
-__device__ __forceinline__ double4 node_vec(const DevModel &M, int field, int i)
+__device__ __forceinline__ double4 node_vec_at(const DevModel &M, int field, int i, int f0)
 {
-  const int inst = (M.nInst > 1) ? find_segment(M.inst_node_begin, M.nInst, i) : 0;
-  const int f0 = M.ctl[inst].f0;
   double4 v = make_double4(0, 0, 0, 0);
   switch (field)
   {
@@ -2858,6 +2864,12 @@ __device__ __forceinline__ double4 node_vec(const DevModel &M, int field, int i)
   default: break;
   }
   return v;
+}
+
+__device__ __forceinline__ double4 node_vec(const DevModel &M, int field, int i)
+{
+  const int inst = (M.nInst > 1) ? find_segment(M.inst_node_begin, M.nInst, i) : 0;
+  return node_vec_at(M, field, i, M.ctl[inst].f0);
 }
 
 // Nodal vector `field` of nodes [n0, n0 + n) as [n][3] FP64 (the layout of
@@ -3026,19 +3038,26 @@ struct HistRing
 };
 
 // Kinetic energy of instance 0 on speed buffer fsel: the loop and tree of
-// k_energies (same order, same bits).  Called by a whole block of 256.
-__device__ __forceinline__ double block_kinetic(const DevModel &M, int fsel, double *sh)
+// k_energies (256 strided sums added as a tree: same order, same bits).
+// Called by a whole block of 256 threads, or of 128 of which each takes two
+// of the sums.
+template <int THREADS> __device__ __forceinline__ double block_kinetic(const DevModel &M, const Ctl &c, int fsel, double *sh)
 {
-  const Ctl &c = M.ctl[0];
-  double ke = 0.0;
-  for (int i = c.node_begin + threadIdx.x; i < c.node_end; i += blockDim.x)
+  static_assert(THREADS == 256 || THREADS == 128, "256 strided sums");
+  double ke[256 / THREADS];
+#pragma unroll
+  for (int j = 0; j < 256 / THREADS; j++)
   {
-    const double4 v = M.v[fsel][i];
-    ke += M.mass[i] * (v.x * v.x + v.y * v.y + v.z * v.z) / 2.0;
+    ke[j] = 0.0;
+    for (int i = c.node_begin + threadIdx.x + j * THREADS; i < c.node_end; i += 256)
+    {
+      const double4 v = M.v[fsel][i];
+      ke[j] += M.mass[i] * (v.x * v.x + v.y * v.y + v.z * v.z) / 2.0;
+    }
   }
-  sh[threadIdx.x] = ke;
+  sh[threadIdx.x] = THREADS == 256 ? ke[0] : ke[0] + ke[256 / THREADS - 1];
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1)
+  for (int s = THREADS / 2; s > 0; s >>= 1)
   {
     if (threadIdx.x < s)
       sh[threadIdx.x] += sh[threadIdx.x + s];
@@ -3047,6 +3066,72 @@ __device__ __forceinline__ double block_kinetic(const DevModel &M, int fsel, dou
   const double r = sh[0];
   __syncthreads();
   return r;
+}
+
+// The schedules due at time t (one thread): the mask, and their next times moved on.
+__device__ __forceinline__ unsigned long long history_due(int nSched, double t, const double *start, double *next,
+                                                          const double *save)
+{
+  unsigned long long mask = 0ull;
+  for (int j = 0; j < nSched; j++)
+    if (!(t > start[j] && t < next[j]))
+    {
+      next[j] += save[j];
+      mask |= 1ull << j;
+    }
+  return mask;
+}
+
+// A slot of the ring for the record of an increment, its header written (one
+// thread); -1 when the ring is full.
+__device__ __forceinline__ int history_slot(const HistRing &H, const Ctl &c, long long inc, unsigned long long mask,
+                                            int nValues)
+{
+  const int k = *H.count;
+  if (k >= H.cap)
+  {
+    *H.overflow = 1;
+    return -1;
+  }
+  *H.count = k + 1;
+  double *r = H.rec + (size_t)k * (HIST_HEAD + nValues);
+  r[0] = c.t;
+  r[1] = (double)inc;
+  r[2] = c.dt_last;
+  r[3] = (double)(unsigned)(mask & 0xffffffffull);
+  r[4] = (double)(unsigned)(mask >> 32);
+  return k;
+}
+
+// The items of a record (a whole block of THREADS).  c: the control block (or a
+// copy) after the end of the increment; sh: THREADS doubles.
+template <typename R, int THREADS>
+__device__ __forceinline__ void history_items(const DevModel &M, const Ctl &c, const int4 *items, const long long *off,
+                                              int nItems, int kin, double *vals, double *sh)
+{
+  double kinv[2] = {0.0, 0.0};
+  if (kin)
+  {
+    kinv[0] = block_kinetic<THREADS>(M, c, c.f0, sh);
+    kinv[1] = block_kinetic<THREADS>(M, c, 1 - c.f0, sh);
+  }
+  for (int k = threadIdx.x; k < nItems; k += THREADS)
+  {
+    const int4 it = items[k];
+    double *o = vals + off[k];
+    if (it.x == DNL_ITEM_POINT)
+      for (int q = 0; q < DNL_IP_NCOMP; q++)
+        o[q] = (double)ipv<R>(M, q, it.z);
+    else if (it.x == DNL_ITEM_KINETIC)
+      o[0] = kinv[it.y == DNL_NODE_SPEED_PREV ? 1 : 0];
+    else
+    {
+      const double4 v = node_vec_at(M, it.y, it.z, c.f0);
+      o[0] = v.x;
+      o[1] = v.y;
+      o[2] = v.z;
+    }
+  }
 }
 
 // One block of 256 after the end of the increment (single models).
@@ -3061,64 +3146,19 @@ __global__ void __launch_bounds__(256) k_history_ring(DevModel M, HistRing H, co
   if (threadIdx.x == 0)
   {
     slot = -1;
-    unsigned long long mask = 0ull;
     const long long committed = c.inc - ((c.prepared && c.active) ? 1 : 0);
     if (committed != *H.last)
     {
       *H.last = committed;
-      const double t = c.t;
-      for (int j = 0; j < H.nSched; j++)
-        if (!(t > H.start[j] && t < H.next[j]))
-        {
-          H.next[j] += H.save[j];
-          mask |= 1ull << j;
-        }
+      const unsigned long long mask = history_due(H.nSched, c.t, H.start, H.next, H.save);
       if (mask)
-      {
-        const int k = *H.count;
-        if (k < H.cap)
-        {
-          slot = k;
-          *H.count = k + 1;
-          double *r = H.rec + (size_t)k * (HIST_HEAD + nValues);
-          r[0] = t;
-          r[1] = (double)committed;
-          r[2] = c.dt_last;
-          r[3] = (double)(unsigned)(mask & 0xffffffffull);
-          r[4] = (double)(unsigned)(mask >> 32);
-        }
-        else
-          *H.overflow = 1;
-      }
+        slot = history_slot(H, c, committed, mask, nValues);
     }
   }
   __syncthreads();
   if (slot < 0)
     return;
-  double kinv[2] = {0.0, 0.0};
-  if (kin)
-  {
-    kinv[0] = block_kinetic(M, c.f0, sh);
-    kinv[1] = block_kinetic(M, 1 - c.f0, sh);
-  }
-  double *vals = H.rec + (size_t)slot * (HIST_HEAD + nValues) + HIST_HEAD;
-  for (int k = threadIdx.x; k < nItems; k += blockDim.x)
-  {
-    const int4 it = items[k];
-    double *o = vals + off[k];
-    if (it.x == DNL_ITEM_POINT)
-      for (int q = 0; q < DNL_IP_NCOMP; q++)
-        o[q] = (double)ipv<R>(M, q, it.z);
-    else if (it.x == DNL_ITEM_KINETIC)
-      o[0] = kinv[it.y == DNL_NODE_SPEED_PREV ? 1 : 0];
-    else
-    {
-      const double4 v = node_vec(M, it.y, it.z);
-      o[0] = v.x;
-      o[1] = v.y;
-      o[2] = v.z;
-    }
-  }
+  history_items<R, 256>(M, c, items, off, nItems, kin, H.rec + (size_t)slot * (HIST_HEAD + nValues) + HIST_HEAD, sh);
 }
 
 // -------------------------------------------------------------- energies

@@ -84,6 +84,7 @@ struct StaticIo
   __device__ __forceinline__ void put(int c, double v) const { ip[(size_t)c * nIP + q] = v; }
   __device__ __forceinline__ void slot(const double4 &v) const { slots[q] = v; }
   __device__ __forceinline__ const float *ip32() const { return nullptr; }
+  __device__ __forceinline__ int ip32_index() const { return q; }
   __device__ __forceinline__ void first_node(unsigned amask, int base, const double4 &X, const double4 &U,
                                              double4 &X0, double4 &U0) const
   {
@@ -236,7 +237,7 @@ template <int NPE> __global__ void __launch_bounds__(TILE) k_sp_element(Args a)
   const int nIP = a.nE * NPE;
   StaticIo io{a.coords, a.du, a.ip, s.slot, s.mat, nIP, q};
   PlainState old{a.ip, nIP, q};
-  element_update<double, NPE>(io, s.ctl, q, e, g, base, amask, a.conn[q], old, sh + threadIdx.x * ROW,
+  element_update<double, NPE>(io, s.ctl, s.ctl, q, e, g, base, amask, a.conn[q], old, sh + threadIdx.x * ROW,
                               sh + (threadIdx.x - g) * ROW);
 }
 

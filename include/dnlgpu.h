@@ -338,7 +338,9 @@ int dnl_engine_energies(dnl_engine *h, int32_t instance, double out[3]);
  * 64 with CUDA events around each pass that are read after the chunk, so
  * that no bracket holds host launch latency; the run stops at the end of
  * the chunk in which its instances stop (the increments past the stop do
- * nothing and add a few microseconds each to the sums). */
+ * nothing and add a few microseconds each to the sums).  A small single model,
+ * whose increments run in one cooperative launch whether timed or not, fills
+ * them from the device's clock at the ends of the launch's phases. */
 int dnl_engine_set_timing(dnl_engine *h, int32_t on);
 int dnl_engine_timings(const dnl_engine *h, double out[4]);
 
@@ -347,7 +349,10 @@ int dnl_engine_timings(const dnl_engine *h, double out[4]);
  * increment's last kernel ends (programmatic serialization inside the graph)
  * instead of after a replay boundary (1.2 % per increment on the
  * 153,600-element bar from 1 to 8).  A run stops on the same increment
- * either way: the increments past an instance's stop do nothing. */
+ * either way: the increments past an instance's stop do nothing.  Small single
+ * models with the Courant time step (FP64 up to 7,104 hexahedra, mixed up to
+ * 9,472) run their increments in cooperative launches instead, unless a
+ * variant was set with dnl_engine_set_variant. */
 int dnl_engine_set_graph_increments(dnl_engine *h, int32_t n);
 
 /* Number of kernel launches issued on the device by the last run call. */
