@@ -2914,53 +2914,111 @@ template <int NPE> __device__ __forceinline__ double extrapolation_weight(int n,
     return m == 2 ? 1.0 + r3 / 2 : m == 1 ? -0.5 : 1.0 - r3 / 2;
 }
 
+// NPE values of component run `comp` of element e's points, as 16-byte loads
+// (an element's points are NPE consecutive values of a run).
+template <typename R, int NPE>
+__device__ __forceinline__ void element_values(const DevModel &M, int comp, int e, R (&v)[NPE])
+{
+  const R *p = reinterpret_cast<const R *>(M.ip) + ip_index(comp, e * NPE);
+  if constexpr (sizeof(R) == 4)
+  {
+#pragma unroll
+    for (int k = 0; k < NPE / 4; k++)
+    {
+      const float4 a = reinterpret_cast<const float4 *>(p)[k];
+      v[4 * k] = a.x;
+      v[4 * k + 1] = a.y;
+      v[4 * k + 2] = a.z;
+      v[4 * k + 3] = a.w;
+    }
+  }
+  else
+  {
+#pragma unroll
+    for (int k = 0; k < NPE / 2; k++)
+    {
+      const double2 a = reinterpret_cast<const double2 *>(p)[k];
+      v[2 * k] = a.x;
+      v[2 * k + 1] = a.y;
+    }
+  }
+}
+
 // Nodal values of point-state quantities as the reference extracts them for
 // its node fields and result files (Node::fieldScalar / fieldSymTensor2,
 // Node.C:244-365): at node i, the sum over its elements (in element order)
 // and their Gauss points of extrapolation_weight * value, divided by the
 // number of elements.  comps.c[j]: a point-state component DNL_IP_*, or
 // DNL_NODE_AVG_VON_MISES (the von Mises stress of each point, dnlVonMises,
-// Macros.h:71).  One thread per (component, node); dst [comps.n][nN].
+// Macros.h:71).  One thread per node and AVG_GROUP components, which share the
+// element list and the weights; dst [comps.n][nN].  Bound by the L2 sectors of
+// the gather.  The call for 22 components of the 153,600-element bar took 3,951
+// us with one value a load and one component a thread and takes 3,581 so, of
+// which about 3,400 are the copy into a fresh host array.
 struct AvgComps
 {
   static constexpr int MAX = 32;
   int n;
   int c[MAX];
 };
+constexpr int AVG_GROUP = 4;
 template <typename R, int NPE>
-__global__ void k_node_average(DevModel M, const int *slot_inc, AvgComps comps, double *dst, const int *perm)
+__global__ void __launch_bounds__(128) k_node_average(DevModel M, const int *slot_inc, AvgComps comps, double *dst,
+                                                      const int *perm)
 {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)comps.n * M.nN)
+  const int i = blockIdx.x * blockDim.x + threadIdx.x; // the caller's node
+  if (i >= M.nN)
     return;
-  const int j = (int)(t / M.nN), i = (int)(t % M.nN); // i: the caller's node
-  const int comp = comps.c[j];
+  const int j0 = blockIdx.y * AVG_GROUP, nj = min(AVG_GROUP, comps.n - j0);
   const int ni = perm ? perm[i] : i;
   const int kb = slot_begin(M, ni), ke = kb + M.csr_off[ni + 1] - M.csr_off[ni];
-  double acc = 0.0;
+  double acc[AVG_GROUP];
+#pragma unroll
+  for (int j = 0; j < AVG_GROUP; j++)
+    acc[j] = 0.0;
   for (int k = kb; k < ke; k++)
   {
     const int inc = slot_inc[k];
     const int e = inc / NPE, loc = inc % NPE;
+    double w[NPE];
 #pragma unroll
     for (int g = 0; g < NPE; g++)
+      w[g] = extrapolation_weight<NPE>(loc, g);
+#pragma unroll
+    for (int j = 0; j < AVG_GROUP; j++)
     {
-      const int q = e * NPE + g;
-      double v;
+      if (j >= nj)
+        break;
+      const int comp = comps.c[j0 + j];
       if (comp == DNL_NODE_AVG_VON_MISES)
       {
-        const double s1 = ipv<R>(M, DNL_IP_STRESS + 0, q), s2 = ipv<R>(M, DNL_IP_STRESS + 3, q),
-                     s3 = ipv<R>(M, DNL_IP_STRESS + 5, q), s4 = ipv<R>(M, DNL_IP_STRESS + 1, q),
-                     s5 = ipv<R>(M, DNL_IP_STRESS + 2, q), s6 = ipv<R>(M, DNL_IP_STRESS + 4, q);
-        v = sqrt(((s1 - s2) * (s1 - s2) + (s1 - s3) * (s1 - s3) + (s2 - s3) * (s2 - s3) +
-                  6.0 * (s4 * s4 + s5 * s5 + s6 * s6)) / 2);
+        R s[6][NPE];
+#pragma unroll
+        for (int c = 0; c < 6; c++)
+          element_values<R, NPE>(M, DNL_IP_STRESS + c, e, s[c]);
+#pragma unroll
+        for (int g = 0; g < NPE; g++)
+        {
+          const double s1 = s[0][g], s2 = s[3][g], s3 = s[5][g], s4 = s[1][g], s5 = s[2][g], s6 = s[4][g];
+          const double v = sqrt(((s1 - s2) * (s1 - s2) + (s1 - s3) * (s1 - s3) + (s2 - s3) * (s2 - s3) +
+                                 6.0 * (s4 * s4 + s5 * s5 + s6 * s6)) / 2);
+          acc[j] = __dadd_rn(acc[j], __dmul_rn(w[g], v));
+        }
       }
       else
-        v = (double)ipv<R>(M, comp, q);
-      acc = __dadd_rn(acc, __dmul_rn(extrapolation_weight<NPE>(loc, g), v));
+      {
+        R v[NPE];
+        element_values<R, NPE>(M, comp, e, v);
+#pragma unroll
+        for (int g = 0; g < NPE; g++)
+          acc[j] = __dadd_rn(acc[j], __dmul_rn(w[g], (double)v[g]));
+      }
     }
   }
-  dst[t] = acc / (double)(ke - kb);
+#pragma unroll
+  for (int j = 0; j < AVG_GROUP; j++)
+    if (j < nj)
+      dst[(size_t)(j0 + j) * M.nN + i] = acc[j] / (double)(ke - kb);
 }
 
 // Components [c0, c0 + nc) of the point state, tile-major in R, to a
@@ -3037,32 +3095,83 @@ struct HistRing
   double *rec;                 // [cap][HIST_HEAD + nValues]
 };
 
-// Kinetic energy of instance 0 on speed buffer fsel: the loop and tree of
-// k_energies (256 strided sums added as a tree: same order, same bits).
-// Called by a whole block of 256 threads, or of 128 of which each takes two
-// of the sums.
-template <int THREADS> __device__ __forceinline__ double block_kinetic(const DevModel &M, const Ctl &c, int fsel, double *sh)
+// Kinetic energy of an instance as a sum of fixed order, whoever computes it:
+// KIN_GROUPS groups of 256 lanes, lane L of all taking the nodes L, L +
+// 256 KIN_GROUPS, ...; the lanes of a warp are added by a butterfly, the warps
+// of a group and then the groups in order.  k_energy_parts has a block per
+// group; the history record's block computes all the groups (block_kinetic).
+constexpr int KIN_GROUPS = 32;
+__device__ __forceinline__ double node_kinetic(const DevModel &M, int fsel, int i)
 {
-  static_assert(THREADS == 256 || THREADS == 128, "256 strided sums");
-  double ke[256 / THREADS];
+  const double4 v = M.v[fsel][i];
+  return __dmul_rn(0.5 * M.mass[i], __fma_rn(v.z, v.z, __fma_rn(v.y, v.y, __dmul_rn(v.x, v.x))));
+}
+__device__ __forceinline__ double warp_sum(double v)
+{
 #pragma unroll
-  for (int j = 0; j < 256 / THREADS; j++)
-  {
-    ke[j] = 0.0;
-    for (int i = c.node_begin + threadIdx.x + j * THREADS; i < c.node_end; i += 256)
+  for (int o = 16; o > 0; o >>= 1)
+    v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+// a group's eight warps in order
+__device__ __forceinline__ double group_total(const double *w)
+{
+  double s = w[0];
+#pragma unroll
+  for (int k = 1; k < 8; k++)
+    s = __dadd_rn(s, w[k]);
+  return s;
+}
+// lane b of a warp holds group b: their sum in order, in every lane
+__device__ __forceinline__ double groups_total(double v)
+{
+  double s = __shfl_sync(0xffffffffu, v, 0);
+  for (int b = 1; b < KIN_GROUPS; b++)
+    s = __dadd_rn(s, __shfl_sync(0xffffffffu, v, b));
+  return s;
+}
+static_assert(KIN_GROUPS == 32, "a lane per group");
+
+// All the groups by one block of THREADS (128 or 256); sh: 8 KIN_GROUPS doubles.
+// GB groups at once keep that many loads in flight.
+template <int THREADS, int GB>
+__device__ __forceinline__ double block_kinetic(const DevModel &M, const Ctl &c, int fsel, double *sh)
+{
+  for (int b0 = 0; b0 < KIN_GROUPS; b0 += GB)
+#pragma unroll 1
+    for (int l0 = threadIdx.x; l0 < 256; l0 += THREADS)
     {
-      const double4 v = M.v[fsel][i];
-      ke[j] += M.mass[i] * (v.x * v.x + v.y * v.y + v.z * v.z) / 2.0;
+      double ke[GB];
+#pragma unroll
+      for (int b = 0; b < GB; b++)
+        ke[b] = 0.0;
+      for (int i0 = c.node_begin + b0 * 256 + l0; i0 < c.node_end; i0 += 256 * KIN_GROUPS)
+      {
+        double k[GB];
+#pragma unroll
+        for (int b = 0; b < GB; b++)
+          k[b] = i0 + 256 * b < c.node_end ? node_kinetic(M, fsel, i0 + 256 * b) : 0.0;
+#pragma unroll
+        for (int b = 0; b < GB; b++)
+          ke[b] = __dadd_rn(ke[b], k[b]);
+      }
+#pragma unroll
+      for (int b = 0; b < GB; b++)
+      {
+        const double w = warp_sum(ke[b]);
+        if ((threadIdx.x & 31) == 0)
+          sh[8 * (b0 + b) + (l0 >> 5)] = w;
+      }
     }
-  }
-  sh[threadIdx.x] = THREADS == 256 ? ke[0] : ke[0] + ke[256 / THREADS - 1];
   __syncthreads();
-  for (int s = THREADS / 2; s > 0; s >>= 1)
+  if (threadIdx.x < 32)
   {
-    if (threadIdx.x < s)
-      sh[threadIdx.x] += sh[threadIdx.x + s];
-    __syncthreads();
+    const double r = groups_total(group_total(sh + 8 * threadIdx.x));
+    __syncwarp();
+    if (threadIdx.x == 0)
+      sh[0] = r;
   }
+  __syncthreads();
   const double r = sh[0];
   __syncthreads();
   return r;
@@ -3104,17 +3213,18 @@ __device__ __forceinline__ int history_slot(const HistRing &H, const Ctl &c, lon
 }
 
 // The items of a record (a whole block of THREADS).  c: the control block (or a
-// copy) after the end of the increment; sh: THREADS doubles.
+// copy) after the end of the increment; kin: the speed buffers whose kinetic
+// energy is asked for (bit 0 current, bit 1 previous); sh: 8 KIN_GROUPS doubles.
 template <typename R, int THREADS>
 __device__ __forceinline__ void history_items(const DevModel &M, const Ctl &c, const int4 *items, const long long *off,
                                               int nItems, int kin, double *vals, double *sh)
 {
   double kinv[2] = {0.0, 0.0};
-  if (kin)
-  {
-    kinv[0] = block_kinetic<THREADS>(M, c, c.f0, sh);
-    kinv[1] = block_kinetic<THREADS>(M, c, 1 - c.f0, sh);
-  }
+  constexpr int GB = THREADS == 256 ? 8 : 2; // k_steps has no registers to spare, and fewer nodes
+  if (kin & 1)
+    kinv[0] = block_kinetic<THREADS, GB>(M, c, c.f0, sh);
+  if (kin & 2)
+    kinv[1] = block_kinetic<THREADS, GB>(M, c, 1 - c.f0, sh);
   for (int k = threadIdx.x; k < nItems; k += THREADS)
   {
     const int4 it = items[k];
@@ -3140,7 +3250,7 @@ __global__ void __launch_bounds__(256) k_history_ring(DevModel M, HistRing H, co
                                                       const long long *off, int nItems, int nValues, int kin)
 {
   pdl_wait();
-  __shared__ double sh[256];
+  __shared__ double sh[8 * KIN_GROUPS];
   __shared__ int slot;
   const Ctl &c = M.ctl[0];
   if (threadIdx.x == 0)
@@ -3163,42 +3273,75 @@ __global__ void __launch_bounds__(256) k_history_ring(DevModel M, HistRing H, co
 
 // -------------------------------------------------------------- energies
 
-// One block per instance, fixed-order tree sums (deterministic).
+// Sums of fixed order (deterministic), spread over the GPU: the partials of an
+// instance (blockIdx.y) by ENERGY_BLOCKS blocks, then their sum by one warp.
+// The points go to 256 ENERGY_BLOCKS lanes as the nodes to the lanes of
+// node_kinetic above.  Bound by the latency of its loads; in one block per
+// instance the call on the 153,600-element bar (1.2 million points) took 2,360
+// us, it takes 41 so.
+constexpr int ENERGY_BLOCKS = 256;
+constexpr int ENERGY_PARTS = KIN_GROUPS + 2 * ENERGY_BLOCKS; // doubles per instance: kinetic | internal | inelastic
 template <typename R, int NPE>
-__global__ void k_energies(DevModel M, double *out /* [nInst*3] */, int speed_field)
+__global__ void __launch_bounds__(256) k_energy_parts(DevModel M, double *part, int speed_field, int points)
 {
-  const int inst = blockIdx.x;
-  const Ctl &c = M.ctl[inst];
-  __shared__ double sh[3][256];
+  __shared__ double sh[3][8];
+  const Ctl &c = M.ctl[blockIdx.y];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, b = blockIdx.x;
+  double *out = part + (size_t)blockIdx.y * ENERGY_PARTS;
   double ke = 0.0, ei = 0.0, ep = 0.0;
-  const int fsel = speed_field ? (1 - c.f0) : c.f0;
-  for (int i = c.node_begin + threadIdx.x; i < c.node_end; i += blockDim.x)
+  if (b < KIN_GROUPS)
   {
-    const double4 v = M.v[fsel][i];
-    ke += M.mass[i] * (v.x * v.x + v.y * v.y + v.z * v.z) / 2.0;
+    const int fsel = speed_field ? (1 - c.f0) : c.f0;
+#pragma unroll 4
+    for (int i = c.node_begin + b * 256 + t; i < c.node_end; i += 256 * KIN_GROUPS)
+      ke = __dadd_rn(ke, node_kinetic(M, fsel, i));
+    ke = warp_sum(ke);
   }
-  const double wfac = (NPE == 4 && !c.plane) ? 6.28318530717958647692 : 1.0;
-  for (int q = c.elem_begin * NPE + threadIdx.x; q < c.elem_end * NPE; q += blockDim.x)
+  if (points)
   {
-    const MatDev &mp = M.mat[M.emat[q / NPE]];
-    const double w = mp.rho0 * (double)ipv<R>(M, DNL_IP_DETJ0, q) * wfac;
-    ei += w * (double)ipv<R>(M, DNL_IP_EINT, q);
-    ep += w * (double)ipv<R>(M, DNL_IP_EINEL, q);
+    const double wfac = (NPE == 4 && !c.plane) ? 6.28318530717958647692 : 1.0;
+#pragma unroll 4
+    for (int q = c.elem_begin * NPE + b * 256 + t; q < c.elem_end * NPE; q += 256 * ENERGY_BLOCKS)
+    {
+      const double wt = M.mat[M.emat[q / NPE]].rho0 * (double)ipv<R>(M, DNL_IP_DETJ0, q) * wfac;
+      ei += wt * (double)ipv<R>(M, DNL_IP_EINT, q);
+      ep += wt * (double)ipv<R>(M, DNL_IP_EINEL, q);
+    }
+    ei = warp_sum(ei);
+    ep = warp_sum(ep);
   }
-  sh[0][threadIdx.x] = ke;
-  sh[1][threadIdx.x] = ei;
-  sh[2][threadIdx.x] = ep;
+  if (lane == 0)
+  {
+    sh[0][w] = ke;
+    sh[1][w] = ei;
+    sh[2][w] = ep;
+  }
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1)
+  if (t < 3 && (t > 0 || b < KIN_GROUPS))
+    out[t == 0 ? b : KIN_GROUPS + (t - 1) * ENERGY_BLOCKS + b] = group_total(sh[t]);
+}
+
+// out: [nInst][3] kinetic, internal, inelastic (points = 0: the kinetic only)
+__global__ void __launch_bounds__(32) k_energy_sum(const double *part, double *out, int points)
+{
+  const double *p = part + (size_t)blockIdx.x * ENERGY_PARTS;
+  const int lane = threadIdx.x;
+  const double ke = groups_total(p[lane]);
+  double e[2] = {0.0, 0.0};
+  if (points)
+    for (int k = 0; k < 2; k++)
+    {
+      const double *q = p + KIN_GROUPS + k * ENERGY_BLOCKS + lane * (ENERGY_BLOCKS / 32);
+      static_assert(ENERGY_BLOCKS / 32 == 8, "eight partials per lane");
+      e[k] = warp_sum(group_total(q));
+    }
+  if (lane == 0)
   {
-    if (threadIdx.x < s)
-      for (int k = 0; k < 3; k++)
-        sh[k][threadIdx.x] += sh[k][threadIdx.x + s];
-    __syncthreads();
+    double *o = out + 3 * (size_t)blockIdx.x;
+    o[0] = ke;
+    o[1] = e[0];
+    o[2] = e[1];
   }
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; k++)
-      out[3 * inst + k] = sh[k][0];
 }
 
 } // namespace

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
   __shared__ Ctl c; // this block's control values
   __shared__ int gaveUp, hslot, hdue;
   __shared__ long long hlast;
-  __shared__ double hsched[3][64], red[TILE];
+  __shared__ double hsched[3][64], red[8 * KIN_GROUPS];
   const int t = threadIdx.x, lane = t & 31;
   if (t == 0)
   {

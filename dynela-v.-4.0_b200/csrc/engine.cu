@@ -46,7 +46,7 @@ struct dnl_engine
   const int *dIntOf = nullptr;
   std::vector<Ctl> ctlInit;
   Ctl *hctl = nullptr; // host mirror of the control blocks
-  double *denergy = nullptr;
+  double *denergy = nullptr, *denergyPart = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graphExec = nullptr;
   // graphs of r < graphIncs increments (remExec[r]), for runs of a known
@@ -80,7 +80,7 @@ struct dnl_engine
   // history items (dnl_engine_set_items): list, output offsets, values
   int nItems = 0;
   long long nValues = 0;
-  bool itemsKinetic = false;
+  int itemsKinetic = 0; // speed buffers whose kinetic energy an item asks for (bit 0 current, bit 1 previous)
   int4 *ditems = nullptr;
   long long *ditemOff = nullptr;
   double *dvalues = nullptr, *dkin = nullptr;
@@ -630,7 +630,7 @@ int launch_history(dnl_engine *h)
 {
   if (!h->histOn)
     return DNL_OK;
-  const int kin = h->itemsKinetic ? 1 : 0;
+  const int kin = h->itemsKinetic;
   if (h->precision == DNL_PREC_MIXED)
     launch_pdl(h, k_history_ring<float>, 1, 256, 0, h->M, h->hist, (const int4 *)h->ditems,
                (const long long *)h->ditemOff, h->nItems, (int)h->nValues, kin);
@@ -727,7 +727,7 @@ int launch_steps(dnl_engine *h, int n, bool timed)
     a.off = h->ditemOff;
     a.nItems = h->nItems;
     a.nValues = (int)h->nValues;
-    a.kin = h->itemsKinetic ? 1 : 0;
+    a.kin = h->itemsKinetic;
   }
   CK(cudaMemsetAsync(h->stepsBar, 0, sizeof(unsigned), h->stream));
   int rc = DNL_STEPS_DISPATCH(launch_steps_t, h, a);
@@ -1037,7 +1037,7 @@ int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_e
                o_mass = reserve(sizeof(double) * nN), o_ctl = reserve(sizeof(Ctl) * nI),
                o_perm = reserve(sizeof(int) * (renum ? nN : 1)),
                // zeroed at creation, from here to o_ip
-               o_energy = reserve(sizeof(double) * 3 * nI), o_err = reserve(sizeof(int)),
+               o_energy = reserve(sizeof(double) * (3 + ENERGY_PARTS) * nI), o_err = reserve(sizeof(int)),
                o_stats = reserve(sizeof(unsigned long long) * 5), o_done = reserve(sizeof(unsigned) * 2),
                o_steps = reserve(sizeof(unsigned long long) * 4),
                o_act = reserve(sizeof(int)), o_actlist = reserve(sizeof(int) * nI),
@@ -1094,6 +1094,7 @@ int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_e
   M.ctl = (Ctl *)(A + o_ctl);
   h->dIntOf = renum ? (const int *)(A + o_perm) : nullptr;
   h->denergy = (double *)(A + o_energy);
+  h->denergyPart = h->denergy + 3 * nI;
   h->derr = (int *)(A + o_err);
   h->dstats = (unsigned long long *)(A + o_stats);
   M.done_count = (unsigned *)(A + o_done);
@@ -1738,16 +1739,15 @@ int node_averages_dev(dnl_engine *h, const int32_t *comps, int n, double *dst)
     ac.n = std::min(AvgComps::MAX, n - b);
     for (int k = 0; k < ac.n; k++)
       ac.c[k] = comps[b + k];
-    const long long items = (long long)ac.n * h->nN;
-    const unsigned blocks = (unsigned)((items + 255) / 256);
+    const dim3 grid((h->nN + 127) / 128, (ac.n + AVG_GROUP - 1) / AVG_GROUP);
     double *o = dst + (size_t)b * h->nN;
     const bool f32 = h->precision == DNL_PREC_MIXED;
     if (h->npe == 8)
-      f32 ? k_node_average<float, 8><<<blocks, 256, 0, h->stream>>>(h->M, h->dslotInc, ac, o, h->dIntOf)
-          : k_node_average<double, 8><<<blocks, 256, 0, h->stream>>>(h->M, h->dslotInc, ac, o, h->dIntOf);
+      f32 ? k_node_average<float, 8><<<grid, 128, 0, h->stream>>>(h->M, h->dslotInc, ac, o, h->dIntOf)
+          : k_node_average<double, 8><<<grid, 128, 0, h->stream>>>(h->M, h->dslotInc, ac, o, h->dIntOf);
     else
-      f32 ? k_node_average<float, 4><<<blocks, 256, 0, h->stream>>>(h->M, h->dslotInc, ac, o, h->dIntOf)
-          : k_node_average<double, 4><<<blocks, 256, 0, h->stream>>>(h->M, h->dslotInc, ac, o, h->dIntOf);
+      f32 ? k_node_average<float, 4><<<grid, 128, 0, h->stream>>>(h->M, h->dslotInc, ac, o, h->dIntOf)
+          : k_node_average<double, 4><<<grid, 128, 0, h->stream>>>(h->M, h->dslotInc, ac, o, h->dIntOf);
     CK(cudaGetLastError());
     h->launches++;
   }
@@ -2020,22 +2020,25 @@ int dnl_engine_set_ips(dnl_engine *h, const double *in)
 
 namespace
 {
-int launch_energies(dnl_engine *h, double *dst, int speed_field)
+// Energies of every instance into dst [nInst][3]; points = 0: the kinetic only.
+int launch_energies(dnl_engine *h, double *dst, int speed_field, int points)
 {
+  const dim3 grid(points ? ENERGY_BLOCKS : KIN_GROUPS, h->nInst);
   if (h->precision == DNL_PREC_MIXED)
   {
     if (h->npe == 8)
-      k_energies<float, 8><<<h->nInst, 256, 0, h->stream>>>(h->M, dst, speed_field);
+      k_energy_parts<float, 8><<<grid, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points);
     else
-      k_energies<float, 4><<<h->nInst, 256, 0, h->stream>>>(h->M, dst, speed_field);
+      k_energy_parts<float, 4><<<grid, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points);
   }
   else
   {
     if (h->npe == 8)
-      k_energies<double, 8><<<h->nInst, 256, 0, h->stream>>>(h->M, dst, speed_field);
+      k_energy_parts<double, 8><<<grid, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points);
     else
-      k_energies<double, 4><<<h->nInst, 256, 0, h->stream>>>(h->M, dst, speed_field);
+      k_energy_parts<double, 4><<<grid, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points);
   }
+  k_energy_sum<<<h->nInst, 32, 0, h->stream>>>(h->denergyPart, dst, points);
   CK(cudaGetLastError());
   return DNL_OK;
 }
@@ -2052,7 +2055,7 @@ void free_items(dnl_engine *h)
   h->dvalues = h->dkin = h->hvalues = nullptr;
   h->nItems = 0;
   h->nValues = 0;
-  h->itemsKinetic = false;
+  h->itemsKinetic = 0;
 }
 } // namespace
 
@@ -2072,7 +2075,7 @@ int dnl_engine_set_items(dnl_engine *h, const dnl_item *items, int32_t n, int64_
   std::vector<int4> it(n);
   std::vector<long long> off(n);
   long long total = 0;
-  bool kin = false;
+  int kin = 0;
   for (int k = 0; k < n; k++)
   {
     const dnl_item &a = items[k];
@@ -2093,7 +2096,7 @@ int dnl_engine_set_items(dnl_engine *h, const dnl_item *items, int32_t n, int64_
       if (a.index < 0 || a.index >= h->nInst || (a.field != DNL_NODE_SPEED && a.field != DNL_NODE_SPEED_PREV))
         return fail(h, DNL_ERR_ARG, "item %d: instance %d / speed field %d invalid", k, a.index, a.field);
       width = 1;
-      kin = true;
+      kin |= a.field == DNL_NODE_SPEED ? 1 : 2;
       break;
     default:
       return fail(h, DNL_ERR_ARG, "item %d: unknown kind %d", k, a.kind);
@@ -2133,8 +2136,9 @@ int dnl_engine_gather_items(dnl_engine *h, double *out)
   {
     // energies of every instance on both speed fields: field0 then field1
     for (int f = 0; f < 2; f++)
-      if ((rc = launch_energies(h, h->dkin + 3 * f * h->nInst, f)))
-        return rc;
+      if ((h->itemsKinetic >> f) & 1)
+        if ((rc = launch_energies(h, h->dkin + 3 * f * h->nInst, f, 0)))
+          return rc;
   }
   const int threads = 128, blocks = (h->nItems + threads - 1) / threads;
   if (h->precision == DNL_PREC_MIXED)
@@ -2228,7 +2232,7 @@ int dnl_engine_energies(dnl_engine *h, int32_t i, double out[3])
 {
   if (!h || !out || i < 0 || i >= h->nInst)
     return DNL_ERR_ARG;
-  int rc = launch_energies(h, h->denergy, 0);
+  int rc = launch_energies(h, h->denergy, 0, 1);
   if (rc)
     return rc;
   CK(cudaMemcpyAsync(out, h->denergy + 3 * i, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
