@@ -28,16 +28,17 @@ constexpr int MAX_ELEMS = DNL_STATIC_MAX_ELEMS;
 constexpr int MAX_NODES = DNL_STATIC_MAX_NODES;
 constexpr int MAX_IPS = MAX_ELEMS * 8;
 
-// layout of the scratch array (byte offsets)
+// layout of the scratch array (byte offsets); the list holds npe entries per
+// node (the usual case), or the incidences of all nodes one after the other
 constexpr size_t OFF_CTL = 0;
 constexpr size_t OFF_SLOT = 256;
 constexpr size_t OFF_COUNT = OFF_SLOT + sizeof(double4) * MAX_IPS;
 constexpr size_t OFF_CURSOR = OFF_COUNT + sizeof(int) * (MAX_NODES + 1);
-constexpr size_t OFF_LIST = OFF_CURSOR + sizeof(int) * MAX_NODES;
-constexpr size_t OFF_MAT = (OFF_LIST + sizeof(int) * MAX_IPS + 255) / 256 * 256;
-constexpr size_t SCRATCH_BYTES = OFF_MAT + sizeof(MatDev);
+constexpr size_t OFF_LIST = (OFF_CURSOR + sizeof(int) * MAX_NODES + 255) / 256 * 256;
+constexpr size_t SCRATCH_BYTES = OFF_LIST + sizeof(int) * 8 * MAX_NODES;
+static_assert(8 * MAX_NODES >= MAX_IPS, "the list holds every incidence");
 
-// The scratch of every call (about 5.3 MB).  Host code only takes its device
+// The scratch of every call (about 6.8 MB).  Host code only takes its device
 // address (cudaGetSymbolAddress); the kernels receive that address.
 static __device__ __align__(256) unsigned char g_scratch[SCRATCH_BYTES];
 
@@ -46,14 +47,13 @@ struct Scratch
   Ctl *ctl;
   double4 *slot;
   int *count, *cursor, *list;
-  MatDev *mat; // the call's material, read by the return from global memory
 };
 
 __host__ __device__ Scratch carve(unsigned char *base)
 {
   return Scratch{reinterpret_cast<Ctl *>(base + OFF_CTL), reinterpret_cast<double4 *>(base + OFF_SLOT),
                  reinterpret_cast<int *>(base + OFF_COUNT), reinterpret_cast<int *>(base + OFF_CURSOR),
-                 reinterpret_cast<int *>(base + OFF_LIST), reinterpret_cast<MatDev *>(base + OFF_MAT)};
+                 reinterpret_cast<int *>(base + OFF_LIST)};
 }
 
 // Caller's arrays: point state component-major [29][n_ips] FP64, nodes [n][3].
@@ -62,7 +62,7 @@ struct StaticIo
   const double *coords, *du;
   double *ip;
   double4 *slots;
-  const MatDev *mat_;
+  const MatDev *mat_; // in the kernel's parameters: the return takes its constants as operands
   int nIP, q;
   __device__ __forceinline__ double4 x(int n) const
   {
@@ -74,10 +74,10 @@ struct StaticIo
   }
   __device__ __forceinline__ const MatDev &mat(int) const { return *mat_; }
   __device__ __forceinline__ const MatDev *matp(int) const { return mat_; }
-  __device__ __forceinline__ JC<double> law(int) const
+  __device__ __forceinline__ JC<double, true> law(int) const
   {
-    JC<double> j;
-    j.load(*mat_);
+    JC<double, true> j;
+    j.q = &mat_->jc64;
     return j;
   }
   __device__ __forceinline__ double rho0(int) const { return mat_->rho0; }
@@ -122,31 +122,48 @@ __global__ void k_sp_clear(Args a)
     c.active = 1;
     c.dt_eff = a.dt;
     *s.ctl = c;
-    *s.mat = a.mat;
   }
   if (i <= a.nN)
     s.count[i] = 0;
 }
 
-// Node slot counts.  The connectivity is the caller's device array: an entry
-// outside [0, n_nodes) is not counted, and the call reports DNL_ERR_ARG with
-// the element in the control block; the kernels after this one then leave at
-// once, so no index taken from the connectivity reaches memory unchecked.
-__global__ void k_sp_count(Args a)
+// Each incidence into its node's list of npe entries, in any order (the gather
+// sorts them).  The connectivity is the caller's device array: an entry outside
+// [0, n_nodes) is not listed, and the call reports DNL_ERR_ARG with the element
+// in the control block; the kernels after this one then leave at once, so no
+// index taken from the connectivity reaches memory unchecked.  A node with more
+// than npe elements sets `resolves`, which this pass has no other use for: the
+// host then assembles through the lists of k_sp_count and the kernels after it.
+__global__ void k_sp_list(Args a)
 {
   Scratch s = carve(a.scratch);
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= a.nE * a.npe)
     return;
   const int n = a.conn[k];
-  if ((unsigned)n < (unsigned)a.nN)
-    atomicAdd(&s.count[n + 1], 1);
-  else
+  if ((unsigned)n >= (unsigned)a.nN)
+  {
     raise_status(s.ctl, DNL_ERR_ARG, k / a.npe);
+    return;
+  }
+  const int p = atomicAdd(&s.count[n], 1);
+  if (p < a.npe)
+    s.list[n * a.npe + p] = k;
+  else
+    s.ctl->resolves = 1;
 }
 
-// true once k_sp_count has found a connectivity entry out of range.  Only
-// k_sp_count sets DNL_ERR_ARG, and it completes before the kernels that test
+// Node slot counts (connectivity checked by k_sp_list).
+__global__ void k_sp_count(Args a)
+{
+  Scratch s = carve(a.scratch);
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < a.nE * a.npe)
+    atomicAdd(&s.count[a.conn[k] + 1], 1);
+}
+
+// true once k_sp_list has found a connectivity entry out of range.  Only
+// k_sp_list sets DNL_ERR_ARG, and it completes before the kernels that test
 // it start, so every thread of a launch reads the same answer (the element
 // kernel may raise other codes while it runs; those do not stop the pass).
 __device__ __forceinline__ bool bad_input(const Scratch &s)
@@ -158,8 +175,6 @@ __device__ __forceinline__ bool bad_input(const Scratch &s)
 __global__ void k_sp_scan(Args a)
 {
   Scratch s = carve(a.scratch);
-  if (bad_input(s))
-    return;
   __shared__ int part[1024];
   const int n = a.nN + 1, t = threadIdx.x, per = (n + blockDim.x - 1) / blockDim.x;
   const int b = t * per, e = min(n, b + per);
@@ -194,7 +209,7 @@ __global__ void k_sp_fill(Args a)
 {
   Scratch s = carve(a.scratch);
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < a.nE * a.npe && !bad_input(s))
+  if (k < a.nE * a.npe)
     s.list[atomicAdd(&s.cursor[a.conn[k]], 1)] = k;
 }
 
@@ -203,7 +218,7 @@ __global__ void k_sp_sort(Args a)
 {
   Scratch s = carve(a.scratch);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.nN || bad_input(s))
+  if (i >= a.nN)
     return;
   int *L = s.list + s.count[i];
   const int n = s.count[i + 1] - s.count[i];
@@ -220,10 +235,10 @@ __global__ void k_sp_sort(Args a)
   }
 }
 
-template <int NPE> __global__ void __launch_bounds__(TILE) k_sp_element(Args a)
+template <int NPE> __global__ void __launch_bounds__(TILE, 4) k_sp_element(const __grid_constant__ Args a)
 {
   constexpr int ROW = ElemShape<NPE>::template pass_row<double>;
-  __shared__ double sh[TILE * ROW];
+  __shared__ __align__(16) double sh[TILE * ROW];
   Scratch s = carve(a.scratch);
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -235,17 +250,66 @@ template <int NPE> __global__ void __launch_bounds__(TILE) k_sp_element(Args a)
   if (!act)
     return;
   const int nIP = a.nE * NPE;
-  StaticIo io{a.coords, a.du, a.ip, s.slot, s.mat, nIP, q};
+  StaticIo io{a.coords, a.du, a.ip, s.slot, &a.mat, nIP, q};
   PlainState old{a.ip, nIP, q};
   element_update<double, NPE>(io, s.ctl, s.ctl, q, e, g, base, amask, a.conn[q], old, sh + threadIdx.x * ROW,
                               sh + (threadIdx.x - g) * ROW);
 }
 
+// Forces of a node from its list of at most NPE incidences, in increasing
+// element order (the reference's assembly order).
+template <int NPE> __global__ void __launch_bounds__(128) k_sp_assemble(Args a)
+{
+  Scratch s = carve(a.scratch);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.nN || bad_input(s) || s.ctl->resolves)
+    return;
+  const int n = s.count[i];
+  int L[NPE];
+#pragma unroll
+  for (int j = 0; j < NPE / 4; j++)
+  {
+    const int4 v = reinterpret_cast<const int4 *>(s.list + (size_t)i * NPE)[j];
+    L[4 * j] = v.x;
+    L[4 * j + 1] = v.y;
+    L[4 * j + 2] = v.z;
+    L[4 * j + 3] = v.w;
+  }
+#pragma unroll
+  for (int j = 0; j < NPE; j++)
+    L[j] = j < n ? L[j] : 0x7fffffff; // past the list, after every incidence
+#pragma unroll
+  for (int r = 0; r < NPE; r++) // odd-even transposition sort
+#pragma unroll
+    for (int j = r & 1; j + 1 < NPE; j += 2)
+    {
+      const int lo = min(L[j], L[j + 1]), hi = max(L[j], L[j + 1]);
+      L[j] = lo;
+      L[j + 1] = hi;
+    }
+  double4 v[NPE];
+#pragma unroll
+  for (int j = 0; j < NPE; j++)
+    v[j] = j < n ? s.slot[L[j]] : make_double4(0, 0, 0, 0);
+  double fx = 0.0, fy = 0.0, fz = 0.0;
+#pragma unroll
+  for (int j = 0; j < NPE; j++)
+  {
+    fx += v[j].x;
+    fy += v[j].y;
+    fz += v[j].z;
+  }
+  a.force[3 * i] = fx;
+  a.force[3 * i + 1] = fy;
+  a.force[3 * i + 2] = fz;
+}
+
+// The same through the lists of k_sp_sort, of any length.
 __global__ void k_sp_gather(Args a)
 {
   Scratch s = carve(a.scratch);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.nN || bad_input(s))
+  if (i >= a.nN)
     return;
   double fx = 0.0, fy = 0.0, fz = 0.0;
   for (int k = s.count[i]; k < s.count[i + 1]; k++)
@@ -336,22 +400,43 @@ extern "C" int dnl_element_pass_static(int32_t elem_type, int32_t n_nodes, int32
   a.mat = make_mat(m);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int nIP = n_elems * npe;
+  // Four launches.  With the incidence lists built by a count, a one-block scan,
+  // a fill and a sort before the element pass, and the material read from global
+  // memory, the call (with a copy of the point state before it) took 242 us on
+  // 16,384 hexahedra, so 182; those kernels now run only for a mesh with a node
+  // of more than npe elements.
   k_sp_clear<<<(n_nodes + 1 + 255) / 256, 256, 0, st>>>(a);
-  k_sp_count<<<(nIP + 255) / 256, 256, 0, st>>>(a);
-  k_sp_scan<<<1, 1024, 0, st>>>(a);
-  k_sp_fill<<<(nIP + 255) / 256, 256, 0, st>>>(a);
-  k_sp_sort<<<(n_nodes + 255) / 256, 256, 0, st>>>(a);
+  k_sp_list<<<(nIP + 255) / 256, 256, 0, st>>>(a);
   if (npe == 8)
+  {
     k_sp_element<8><<<(nIP + TILE - 1) / TILE, TILE, 0, st>>>(a);
+    k_sp_assemble<8><<<(n_nodes + 127) / 128, 128, 0, st>>>(a);
+  }
   else
+  {
     k_sp_element<4><<<(nIP + TILE - 1) / TILE, TILE, 0, st>>>(a);
-  k_sp_gather<<<(n_nodes + 255) / 256, 256, 0, st>>>(a);
+    k_sp_assemble<4><<<(n_nodes + 127) / 128, 128, 0, st>>>(a);
+  }
   cudaError_t e = cudaGetLastError();
-  int status = 0;
+  Ctl done;
+  done.status = done.resolves = 0;
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&status, &carve(scratch).ctl->status, sizeof(int), cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync(&done, carve(scratch).ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess)
     e = cudaStreamSynchronize(st);
+  const int status = done.status;
+  if (e == cudaSuccess && status != DNL_ERR_ARG && done.resolves)
+  {
+    k_sp_clear<<<(n_nodes + 1 + 255) / 256, 256, 0, st>>>(a);
+    k_sp_count<<<(nIP + 255) / 256, 256, 0, st>>>(a);
+    k_sp_scan<<<1, 1024, 0, st>>>(a);
+    k_sp_fill<<<(nIP + 255) / 256, 256, 0, st>>>(a);
+    k_sp_sort<<<(n_nodes + 255) / 256, 256, 0, st>>>(a);
+    k_sp_gather<<<(n_nodes + 255) / 256, 256, 0, st>>>(a);
+    e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = cudaStreamSynchronize(st);
+  }
   if (e != cudaSuccess)
   {
     snprintf(buf, sizeof(buf), "dnl_element_pass_static: %s", cudaGetErrorString(e));

@@ -387,7 +387,7 @@ const char *dnl_variant_name(int32_t precision, int32_t variant);
  * an allocation would synchronize the device): every input and output is a
  * caller-owned device array, and the scratch (per element-node force slots,
  * node -> slot lists, a control block) is a static device array of about
- * 5.3 MB that every GPU loading the library keeps until the process exits.
+ * 6.8 MB that every GPU loading the library keeps until the process exits.
  * One call = strains, pressure, radial return, final rotation, density and the
  * nodal internal forces (the same element pass as dnl_engine_element_pass) in
  * FP64 for a model of at most DNL_STATIC_MAX_ELEMS elements and
