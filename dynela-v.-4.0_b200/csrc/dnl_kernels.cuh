@@ -390,8 +390,8 @@ template <int NPE> struct ElemShape
   static constexpr int ROW = (NPE * DIM > 18 ? NPE * DIM : 18) + 1;
   // the element pass's row: the rotation and J^-1 parked across the return as
   // 16-byte vectors (the hexahedron's forces need no transpose, the
-  // quadrilaterals' 8 fit).  A row of 20 floats (80 B) or 22 doubles (176 B)
-  // is an odd number of 16-byte units, so the 8 lanes of each phase of a
+  // quadrilaterals' 8 fit), and in FP64 most of the strain increment.  A row of
+  // 20 floats (80 B) or 22 doubles (176 B) is an odd number of 16-byte units, so the 8 lanes of each phase of a
   // 16-byte access reach 8 different bank groups
   template <typename R> static constexpr int pass_row = sizeof(R) == 4 ? 20 : 22;
 };
@@ -964,7 +964,7 @@ __device__ __forceinline__ void element_update(const Io &io, const Ctl *C, Ctl *
   st.pressure = (st.s[0] + st.s[3] + st.s[5]) / R(3) + jc.K() * (trSum / R(NPE));
   {
     bool ok;
-    radial_return<R>(jc, jc.twoG(), jc.heatFrac(), jc.invRho0(), dE, R(dt), st, ok, R(-1), C->direct != 0);
+    radial_return<R>(jc, jc.twoG(), jc.heatFrac(), jc.invRho0(), dE, R(dt), st, ok, R(-1), C->direct != 0, row + 18);
     if (!ok)
     {
       if constexpr (sizeof(R) == 4)
