@@ -286,7 +286,8 @@ __device__ __noinline__ Resolved resolve_fp64(const float *ip, int q, const MatD
   d.pressure = pressure;
   const double de[6] = {e0, e1, e2, e3, e4, e5};
   bool ok;
-  radial_return<double>(jc, mp.twoG, mp.heatFrac, 1.0 / mp.rho0, de, dt, d, ok);
+  // (rarely called: iterates by pow and log take fewer registers around the call)
+  radial_return<double, false>(jc, mp.twoG, mp.heatFrac, 1.0 / mp.rho0, de, dt, d, ok);
   Resolved r;
   for (int c = 0; c < 6; c++)
     r.s[c] = (float)d.s[c];

@@ -404,36 +404,55 @@ inline MatDev make_mat(const dnl_material &m)
   return d;
 }
 
-// (1 + x)^a - 1 for |x| <= 2^-6: the binomial series, nested,
-// a x (1 + (a-1)/2 x (1 + (a-2)/3 x (...))), to a remainder below 2^-58 for
-// exponents of a few units.
-__device__ __forceinline__ double pow1p_m1(double x, double a)
+// Double-precision logarithm and exponential as straight-line code, so that the
+// two powers and the logarithm of the Johnson-Cook law, which do not depend on
+// each other, run as interleaved chains instead of as three calls one after the
+// other.  Method: x = 2^e m with m in [sqrt(1/2), sqrt(2)), s = (m - 1) / (m + 1)
+// and log m = 2 atanh(s) by its Taylor series (Abramowitz and Stegun, Handbook
+// of Mathematical Functions, 4.1.28 and 4.6.33), the leading part as an unevaluated sum of two
+// doubles; exp by reduction modulo ln 2 and the Taylor series on |r| <= ln(2)/2.
+// x^y = exp(y log x) is within 1.01 ulp for x in 1e-18..100 and y in 0..3 (6
+// million random pairs against 113-bit values, mean 0.26; CUDA states 2 ulp for
+// pow), the logarithm within 0.55 ulp.
+struct TwoDoubles
 {
-  const double a1 = a + 1.0;
-  double t = 1.0;
-#pragma unroll
-  for (int k = 9; k >= 2; k--)
-    t = fma(fma(a1, 1.0 / k, -1.0) * x, t, 1.0);
-  return a * x * t;
-}
-// log(1 + x) for |x| <= 1/8: 2 atanh(z), z = x / (2 + x), to z^16 / 17 < 2^-69
-__device__ __forceinline__ double log1p_near(double x)
-{
-  const double z = x / (2.0 + x), z2 = z * z;
-  double t = 1.0 / 15.0;
-#pragma unroll
-  for (int k = 6; k >= 1; k--)
-    t = fma(t, z2, 1.0 / (2 * k + 1));
-  return 2.0 * fma(z * z2, t, z);
-}
-
-// What the law at one iterate of a point's FP64 return leaves for the next.
-struct NearLaw
-{
-  double T;              // temperature
-  double pn, lg, thm;    // epsp^n, ln(depsp / depsp0), th^m (th: the homologous temperature)
-  double re, rg, rt;     // 1 / epsp, 1 / (sqrt(2/3) gamma), 1 / (T - Tref)
+  double hi, lo;
 };
+constexpr double LN2_HI = 0x1.62e42fefa38p-1;    // ln 2 to 42 bits: its products with an exponent are exact
+constexpr double LN2_LO = 0x1.ef35793c7673p-45;  // the rest
+// log x of a positive normal x
+__device__ __forceinline__ TwoDoubles log_two(double x)
+{
+  const int hi = __double2hiint(x), e = (hi - 0x3fe6a09e) >> 20; // high word of sqrt(1/2)
+  const double m = __hiloint2double(hi - (e << 20), __double2loint(x));
+  const double a = m - 1.0, b = m + 1.0, bl = m - (b - 1.0);
+  const double r = 1.0 / b, s = a * r, sl = fma(-s, bl, fma(-s, b, a)) * r;
+  const double z = s * s, z2 = z * z;
+  // 2 s + 2 s z (1/3 + z/5 + ... + z^10/23)
+  const double qe = fma(fma(fma(fma(fma(1.0 / 23, z2, 1.0 / 19), z2, 1.0 / 15), z2, 1.0 / 11), z2, 1.0 / 7), z2, 1.0 / 3);
+  const double qo = fma(fma(fma(fma(1.0 / 21, z2, 1.0 / 17), z2, 1.0 / 13), z2, 1.0 / 9), z2, 1.0 / 5);
+  const double ed = e, eh = ed * LN2_HI, s2 = 2.0 * s, h = __dadd_rn(eh, s2);
+  const double l = __dadd_rn(s2, -__dadd_rn(h, -eh)) + fma(ed, LN2_LO, fma(s2 * z, fma(qo, z, qe), 2.0 * sl));
+  TwoDoubles o;
+  o.hi = __dadd_rn(h, l);
+  o.lo = __dadd_rn(l, -__dadd_rn(o.hi, -h));
+  return o;
+}
+// exp(hi + lo); 0 below the normal range, infinity above it
+__device__ __forceinline__ double exp_two(double hi, double lo)
+{
+  const double k = rint(hi * 1.4426950408889634074);
+  const double rh = fma(-k, LN2_HI, hi), c = fma(-k, LN2_LO, lo);
+  const double r = __dadd_rn(rh, c), rl = __dadd_rn(c, -__dadd_rn(r, -rh)), r2 = r * r;
+  const double pe =
+      fma(fma(fma(fma(fma(1.0 / 479001600, r2, 1.0 / 3628800), r2, 1.0 / 40320), r2, 1.0 / 720), r2, 1.0 / 24), r2, 0.5);
+  const double po = fma(fma(fma(fma(fma(1.0 / 6227020800.0, r2, 1.0 / 39916800), r2, 1.0 / 362880), r2, 1.0 / 5040), r2,
+                            1.0 / 120), r2, 1.0 / 6);
+  const double p = fma(r2, fma(po, r, pe), r); // exp(r) - 1
+  const double v = 1.0 + (p + fma(p, rl, rl));
+  const double w = __hiloint2double(__double2hiint(v) + ((int)k << 20), __double2loint(v));
+  return hi < -708.0 ? 0.0 : (hi > 709.0 ? __longlong_as_double(0x7ff0000000000000ll) : w);
+}
 
 // The Johnson-Cook law as the return calls it.  The parameters are read from
 // the material at each use instead of being held in registers through the
@@ -494,61 +513,40 @@ template <typename R, bool PARAM = false> struct JC
       hard = h;
     }
   }
-  // eval (yield stress and slope) at the iterate gamma of an FP64 return, dg
-  // away from the one before: epsp = epsp0 + sqrt(2/3) gamma, depsp = sqrt(2/3)
-  // gamma / dt.  Two pow and one log of double precision cost most of an
-  // evaluation, and the iterates of a point are close to each other: from the
-  // second on the powers and the logarithm are those at the iterate before
-  // times (plus) a short series in the relative change, exact to the rounding of
-  // that product; where the change is not small (first yield, a bisection from
-  // far) they are evaluated anew.  The reciprocals of an iterate serve its
-  // slope and the next one's changes; neither enters the yield stress other
-  // than times a small change.  Per increment, every iterate evaluated anew ->
-  // so: 800 quads (k_steps) 12.1 -> 10.6 us, 6,048 hexahedra 20.2 -> 16.0,
-  // 153,600 hexahedra 171.5 -> 168.4 (late in 300 increments; the pass is bound
-  // by memory there), 16,384 hexahedra of random plastic states 182 -> 145.
-  __device__ __forceinline__ void eval_near(bool first, double epsp0, double gamma, double dg, double T, double dt,
-                                            NearLaw &c, double &yield, double &hard) const
+  // eval (yield stress and slope) at an iterate of an FP64 return: epsp =
+  // epsp0 + ep, depsp = ep inv_dt, ep = sqrt(2/3) gamma.  An iteration is a chain
+  // of latencies (a warp or two per scheduler in a small model, four in a
+  // large one): with pow, pow and log called one after the other it took about
+  // 3,000 cycles, so about 1,300; the slope's reciprocals do not wait for the
+  // powers.  Per increment, calls -> so: 800 quads in k_steps 17.9 -> 13.1 us
+  // while the front passes and 14.5 -> 11.8 after it, 6,048 hexahedra 23.7 ->
+  // 16.8, 153,600 hexahedra (four warps a scheduler, memory) 171 -> 159; element
+  // pass on 16,384 hexahedra of random plastic states 182 -> 144.  (Following
+  // the powers from one iterate to the next by a series in the change instead
+  // saved less: some lane of nearly every warp had to call.)
+  __device__ __forceinline__ void eval64(double epsp, double ep, double T, double inv_dt, double &yield, double &hard) const
   {
-    const double SQ23 = 0.81649658092772603273;
-    const double ep = SQ23 * gamma, epsp = epsp0 + ep, dep = SQ23 * dg;
-    const double x = dep * c.re;
-    if (!first && fabs(x) <= 0x1p-6)
-      c.pn = fma(c.pn, pow1p_m1(x, ld(q->n)), c.pn);
-    else
-      c.pn = pow(epsp, ld(q->n));
-    const double hard0 = ld(q->A) + ld(q->B) * c.pn;
-    const double depsp = ep / dt;
-    const bool rate = depsp > ld(q->depsp0);
-    const double y = dep * c.rg;
-    if (!first && fabs(y) <= 0.125)
-      c.lg += log1p_near(y);
-    else
-      c.lg = log(depsp / ld(q->depsp0));
-    const double visc0 = rate ? 1.0 + ld(q->C) * c.lg : 1.0;
-    const bool hot = T > ld(q->Tref), warm = hot && T < ld(q->Tm); // warm: neither cold nor molten
-    if (warm)
-    {
-      const double z = (T - c.T) * c.rt; // rt = 0 after an iterate that was not warm
-      if (!first && c.rt != 0.0 && fabs(z) <= 0x1p-6)
-        c.thm = fma(c.thm, pow1p_m1(z, ld(q->m)), c.thm);
-      else
-        c.thm = pow((T - ld(q->Tref)) * ld(q->invTmT), ld(q->m));
-      c.rt = 1.0 / (T - ld(q->Tref));
-    }
-    else
-      c.rt = 0.0;
-    c.T = T;
-    const double temp0 = warm ? 1.0 - c.thm : (hot ? 0.0 : 1.0);
-    c.re = 1.0 / epsp;
-    c.rg = 1.0 / ep;
+    const double n = ld(q->n), m = ld(q->m), dT = T - ld(q->Tref);
+    const bool rate = ep * inv_dt > ld(q->depsp0), hot = dT > 0.0, warm = hot && T < ld(q->Tm); // warm: neither cold nor molten
+    const double re = 1.0 / epsp, rg = 1.0 / ep, rt = 1.0 / dT;
+    const TwoDoubles le = log_two(epsp), lr = log_two(ep * inv_dt / ld(q->depsp0)),
+                     lt = log_two(warm ? dT * ld(q->invTmT) : 1.0);
+    const double eh = n * le.hi, th = m * lt.hi;
+    double pn = exp_two(eh, fma(n, le.lo, fma(n, le.hi, -eh)));
+    const double thm = exp_two(th, fma(m, lt.lo, fma(m, lt.hi, -th)));
+    if (!(epsp >= 0x1p-1022)) // zero, or what the power has no value for
+      pn = epsp >= 0.0 ? (n > 0.0 ? 0.0 : (n == 0.0 ? 1.0 : __longlong_as_double(0x7ff0000000000000ll)))
+                       : __longlong_as_double(0x7ff8000000000000ll);
+    const double hard0 = ld(q->A) + ld(q->B) * pn;
+    const double visc0 = rate ? 1.0 + ld(q->C) * lr.hi : 1.0;
+    const double temp0 = warm ? 1.0 - thm : (hot ? 0.0 : 1.0);
     const double hv = hard0 * visc0;
     yield = hv * temp0;
-    double h = ld(q->n) * ld(q->B) * (epsp > 0.0 ? c.pn * c.re : 0.0) * visc0 * temp0;
+    double h = n * ld(q->B) * (epsp > 0.0 ? pn * re : 0.0) * visc0 * temp0;
     if (rate)
-      h += hard0 * ld(q->C) * temp0 * c.rg;
+      h += hard0 * ld(q->C) * temp0 * rg;
     if (warm)
-      h -= ld(q->m) * ld(q->thermal) * hv * hv * temp0 * c.thm * c.rt;
+      h -= m * ld(q->thermal) * hv * hv * temp0 * thm * rt;
     hard = h;
   }
 };
@@ -602,7 +600,8 @@ __device__ __forceinline__ void trial_state(const Law &jc, R twoG, const R dE[6]
 // gamma = (|s*| - sqrt(2/3) sigma_y) / (2G (1 + h / (3G))) with the slope h at
 // the previous plastic strain (or 1e-8) and rate and the initial temperature,
 // then the yield stress at the new state (1 evaluation).
-template <typename R, class Law>
+// INLINE (FP64): iterates by eval64.
+template <typename R, bool INLINE = sizeof(R) == 8, class Law>
 __device__ __forceinline__ int radial_return(const Law &jc, R twoG, R heatFrac, R inv_rho0, const R dE[6], R dt,
                                              ReturnState<R> &st, bool &ok, R gamma0 = R(-1), bool direct = false,
                                              R *park = nullptr)
@@ -689,13 +688,12 @@ __device__ __forceinline__ int radial_return(const Law &jc, R twoG, R heatFrac, 
     T = T0 + R(0.5) * gamma * heatFrac * (SQ23 * yield + Snorm0);
     R fun = R(0), dfun = twoG32, tol = R(1e-8);
     bool bisected = false; // the last step halved the bracket instead of a Newton step
-    NearLaw near{};        // FP64: the law at the iterate before, and how far it was
-    double dg = 0.0;
+    const R inv_dt = R(1) / dt;
     for (;;)
     {
       R hard;
-      if constexpr (fp64)
-        jc.eval_near(iterate == 0, epsp0, gamma, dg, T, dt, near, yield, hard);
+      if constexpr (INLINE)
+        jc.eval64(epsp, SQ23 * gamma, T, inv_dt, yield, hard);
       else
         jc.eval(epsp, depsp, T, dt, yield, hard, true);
       fun = Strial - gamma * twoG32 - yield;
@@ -705,8 +703,6 @@ __device__ __forceinline__ int radial_return(const Law &jc, R twoG, R heatFrac, 
         gammaMin = gamma;
       dfun = twoG32 + SQ23 * hard;
       R dgamma = fun / dfun;
-      if constexpr (fp64)
-        dg = gamma; // the iterate being left
       gamma += dgamma;
       bisected = (gammaMax - gamma) * (gamma - gammaMin) < R(0);
       if (bisected)
@@ -718,8 +714,6 @@ __device__ __forceinline__ int radial_return(const Law &jc, R twoG, R heatFrac, 
       tol = (fp64 || tolRel < R(1e-8)) ? R(1e-8) : tolRel;
       if (Num<R>::abs_(dgamma) < tol)
         break;
-      if constexpr (fp64)
-        dg = gamma - dg;
       depsp = SQ23 * gamma / dt;
       epsp = epsp0 + SQ23 * gamma;
       T = T0 + R(0.5) * gamma * heatFrac * (SQ23 * yield + Snorm0);

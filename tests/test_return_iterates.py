@@ -1,7 +1,8 @@
-"""The FP64 return evaluates the law at an iterate from the one before when
-the change is small (2^-6 of the plastic strain and the temperature, 1/8 of the
-rate): starts below, around and far above those limits, first yield, cold
-points and points about to melt, against the C restatement."""
+"""The FP64 return evaluates the Johnson-Cook law by its own straight-line
+logarithm and exponential (JC::eval64): starts below, near and far above the
+root, plastic strains over six decades and first yield, cold points, points at
+the reference temperature and about to melt, against the C restatement (libm's
+pow and log)."""
 import numpy as np
 import pytest
 
