@@ -2416,14 +2416,14 @@ __global__ void __launch_bounds__(256) k_courant_finish(DevModel M)
 // applied without forming K_e): eps = B v (Voigt, engineering shear), sig = C eps
 // with the Hooke matrices of Material.C:98-152 (shear modulus term E/(1+nu)),
 // y_n = B_n^T sig w detJ (x 2 pi r, + the hoop row for axisymmetric elements).
-template <int NPE>
-__device__ __forceinline__ void element_Kv(const DevModel &M, int q, int e, int g, int base, unsigned amask,
-                                           const double *v, double scale, double *row, double *grp)
+// row, grp: rows of ROW doubles, the lane's and the element's first.
+template <int NPE, int ROW>
+__device__ __forceinline__ double4 element_Kv(const DevModel &M, int node, int e, int g, int base, unsigned amask,
+                                              bool plane, const double *v, double scale, double *row, const double *grp)
 {
   constexpr int DIM = ElemShape<NPE>::DIM;
-  const bool AXI = ElemShape<NPE>::AXI && !M.ctl[0].plane;
-  constexpr int ROW = ElemShape<NPE>::ROW;
-  const int node = M.conn[q];
+  const bool AXI = ElemShape<NPE>::AXI && !plane;
+  static_assert(ROW >= NPE * DIM, "the transpose needs NPE * DIM values per row");
   const MatDev &mp = M.mat[M.emat[e]];
   double detJ, inv[3][3], radius, H[9];
   const double4 Xn = M.x[node], Un = make_double4(0, 0, 0, 0);
@@ -2527,7 +2527,7 @@ __device__ __forceinline__ void element_Kv(const DevModel &M, int q, int e, int 
     if constexpr (DIM == 3)
       y.z += grp[l * ROW + g * DIM + 2];
   }
-  M.pislot[M.slot_pos[q]] = y;
+  return y;
 }
 
 // Model::computePowerIterationTimeStep (Model.C:942-1009) for a single model,
@@ -2564,7 +2564,8 @@ __global__ void __launch_bounds__(TILE) k_power_iteration(DevModel M, int force)
       const bool act = e < M.nE;
       const unsigned amask = __ballot_sync(0xffffffffu, act);
       if (act)
-        element_Kv<NPE>(M, q, e, g, base, amask, v, scale, sh + t * ROW, sh + (t - g) * ROW);
+        M.pislot[M.slot_pos[q]] = element_Kv<NPE, ROW>(M, M.conn[q], e, g, base, amask, C->plane != 0, v, scale,
+                                                       sh + t * ROW, sh + (t - g) * ROW);
       __syncwarp();
     }
     grid.sync();

@@ -26,6 +26,7 @@ struct StepsArgs
   int nIncs;                // increments of this launch at most
   unsigned *bar;            // arrivals at the grid barrier, zero at launch
   int *err;
+  unsigned long long *pimax; // [3] power iteration: max |v| of an iteration, zero at launch (double bits)
   unsigned long long *phase; // [3] ns spent in the element, nodal and time-step phases, or nullptr
   // history records (dnl_engine_set_history), histOn = 0: none
   int histOn, nItems, nValues, kin;
@@ -125,12 +126,118 @@ template <typename R, bool ONE> struct ResidentIo
   }
 };
 
-template <typename R, int NPE> struct StepsLayout
+template <typename R, int NPE, bool PI> struct StepsLayout
 {
-  static constexpr uint32_t ROW_BYTES = TILE * ElemShape<NPE>::template pass_row<R> * sizeof(R);
+  static constexpr uint32_t PASS_BYTES = TILE * ElemShape<NPE>::template pass_row<R> * sizeof(R);
+  // the power iteration's transpose takes the same rows
+  static constexpr int KV_ROW = NPE == 8 ? 25 : 9;
+  static constexpr uint32_t KV_BYTES = PI ? TILE * KV_ROW * sizeof(double) : 0;
+  static constexpr uint32_t ROW_BYTES = PASS_BYTES > KV_BYTES ? PASS_BYTES : KV_BYTES;
   static constexpr uint32_t STATE_BYTES = DNL_IP_NCOMP * TILE * sizeof(R);
   static_assert(ROW_BYTES % 16 == 0, "the state after the rows is 16-byte aligned");
 };
+
+// State of the power iteration between the time steps of a launch: iterations
+// so far, which buffer holds the vector (M.pv or M.pv2), and the factor that
+// normalises it.
+struct PowerState
+{
+  unsigned it;
+  int odd;
+  double scale;
+};
+
+// k_power_iteration (same sums, same tests) inside the launch: per iteration an
+// element phase and a node phase with a grid barrier after each; the largest
+// |v| of an iteration collects in one of three words, of which the first block
+// clears the next while no block reads it (k_power_iteration has every thread
+// read a word per block).  800 axisymmetric quads with the time step at every
+// increment, per increment, its own launch -> here: 35 -> 19 us (FP64), 24 ->
+// 14 (mixed).  False when a barrier gave up.
+template <typename R, int NPE>
+__device__ __forceinline__ bool power_iteration(const DevModel &M, const StepsArgs &A, Ctl &c, GridBarrier &bar,
+                                                PowerState &pi, double *rows, int t, int node, int spos)
+{
+  constexpr int DIM = ElemShape<NPE>::DIM, ROW = StepsLayout<R, NPE, true>::KV_ROW;
+  const int lane = t & 31, g = t & (NPE - 1), base = lane & ~(NPE - 1);
+  const int e = (blockIdx.x * TILE + t) / NPE;
+  const bool act = e < M.nE;
+  const unsigned amask = __ballot_sync(0xffffffffu, act);
+  double fprev = c.pi_fmax, fmx = 0.0;
+  for (int it = 1;; it++, pi.it++)
+  {
+    const double *v = pi.odd ? M.pv2 : M.pv;
+    double *vn = pi.odd ? M.pv : M.pv2;
+    if (act)
+    {
+      __syncwarp(amask); // the rows of the iteration before have been read
+      M.pislot[spos] = element_Kv<NPE, ROW>(M, node, e, g, base, amask, c.plane != 0, v, pi.scale, rows + t * ROW,
+                                            rows + (t - g) * ROW);
+    }
+    if (blockIdx.x == 0 && t == 0)
+      A.pimax[(pi.it + 1) % 3] = 0ull;
+    if (!bar.sync())
+      return false;
+    double lmax = 0.0;
+    for (int k = blockIdx.x * TILE + t; k < 3 * M.nN; k += gridDim.x * TILE)
+    {
+      const int i = k / 3, cc = k % 3;
+      double val = 0.0;
+      if (cc < DIM)
+      {
+        const double *sl = reinterpret_cast<const double *>(M.pislot) + cc;
+        const int kb = slot_begin(M, i), n = M.csr_off[i + 1] - M.csr_off[i];
+        double acc = v[k] * pi.scale;
+        for (int j0 = 0; j0 < n; j0 += NPE)
+        {
+          double y[NPE];
+#pragma unroll
+          for (int j = 0; j < NPE; j++)
+            y[j] = j0 + j < n ? sl[4 * (size_t)(kb + j0 + j)] : 0.0;
+#pragma unroll
+          for (int j = 0; j < NPE; j++)
+            if (j0 + j < n)
+              acc += y[j];
+        }
+        val = acc / M.mass[i];
+      }
+      vn[k] = val;
+      lmax = fmax(lmax, fabs(val));
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+      lmax = fmax(lmax, __shfl_xor_sync(0xffffffffu, lmax, off));
+    if (lane == 0)
+      atomicMax(&A.pimax[pi.it % 3], (unsigned long long)__double_as_longlong(lmax));
+    if (!bar.sync())
+      return false;
+    fmx = __longlong_as_double((long long)*(volatile unsigned long long *)&A.pimax[pi.it % 3]);
+    const bool conv = fabs(fmx - fprev) / fmx < 1e-4;
+    fprev = fmx;
+    pi.scale = 1.0 / fmx;
+    pi.odd ^= 1;
+    if (conv || it > 1000)
+    {
+      pi.it++;
+      if (t == 0)
+      {
+        if (conv)
+        {
+          c.pi_fmax = fmx;
+          c.pi_omega = sqrt(fmx);
+          c.pi_iters += it;
+        }
+        else
+        {
+          c.status = DNL_ERR_POWER_ITERATION;
+          if (blockIdx.x == 0)
+            raise_status(M.ctl, DNL_ERR_POWER_ITERATION, it);
+        }
+      }
+      return true;
+    }
+  }
+}
 
 // One tile per block, its point state in shared memory from the first
 // increment of the launch to the last.  Bound by latencies: the return's
@@ -141,12 +248,12 @@ template <typename R, int NPE> struct StepsLayout
 // 11.1 -> 7.4 (mixed), 7,747 plane quads 10.7 -> 7.7 (mixed), 6,048 hexahedra
 // 21.1 -> 20.3 (FP64) and 12.8 -> 9.6 (mixed), 8,960 hexahedra 12.7 -> 11.7
 // (mixed).
-template <typename R, int NPE, int MINB, bool ONE>
+template <typename R, int NPE, int MINB, bool ONE, bool PI>
 __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
 {
   constexpr int ROW = ElemShape<NPE>::template pass_row<R>;
   constexpr int DIM = ElemShape<NPE>::DIM;
-  using L = StepsLayout<R, NPE>;
+  using L = StepsLayout<R, NPE, PI>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R *rows = reinterpret_cast<R *>(smem_raw);
   R *st = reinterpret_cast<R *>(smem_raw + L::ROW_BYTES);
@@ -183,6 +290,7 @@ __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
   const bool stamp = A.phase && blockIdx.x == 0 && t == 0;
   unsigned long long ns[3] = {0, 0, 0}, t0 = 0, t1 = 0;
   bool ok = true, reset_min = false;
+  PowerState pi{0, 0, 1.0};
   int done = 0;
   for (; done < A.nIncs && c.active && ok; done++)
   {
@@ -238,7 +346,17 @@ __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
       ns[1] += t0 - t1;
     }
     // ---- time step when due, end of the increment
-    if (due)
+    if constexpr (PI)
+    {
+      if (due)
+      {
+        if (!(ok = power_iteration<R, NPE>(M, A, c, bar, pi, reinterpret_cast<double *>(rows), te, node, spos)))
+          break;
+        if (t == 0 && c.status)
+          status = c.status;
+      }
+    }
+    else if (due)
     {
       const int nE32 = (M.nE + 31) & ~31;
       for (int e = blockIdx.x * TILE + t; e < nE32; e += gridDim.x * TILE)
@@ -289,6 +407,14 @@ __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
     state_out();
   if (reset_min)
     bar.sync(); // every block has read the last minimum
+  if constexpr (PI)
+    if (pi.it)
+    {
+      // the normalised vector for the next launch (M.pv), by the threads that wrote it
+      const double *v = pi.odd ? M.pv2 : M.pv;
+      for (int k = blockIdx.x * TILE + t; k < 3 * M.nN; k += gridDim.x * TILE)
+        M.pv[k] = v[k] * pi.scale;
+    }
   if (blockIdx.x == 0 && t == 0 && done)
   {
     Ctl &G = *M.ctl; // status, bad and resolves are the global block's own
@@ -304,6 +430,9 @@ __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
     G.dt_last = c.dt_last;
     if (reset_min)
       G.min_bits = INF_BITS;
+    G.pi_fmax = c.pi_fmax;
+    G.pi_omega = c.pi_omega;
+    G.pi_iters = c.pi_iters;
     if (A.histOn)
     {
       *A.hist.last = hlast;

@@ -643,10 +643,10 @@ int launch_history(dnl_engine *h)
 
 // Register budgets of k_steps, as blocks per SM: the fewest blocks (most
 // registers) that hold the model's tiles, one per block.
-template <typename R, int NPE, bool ONE, int MINB> int plan_steps_minb(dnl_engine *h)
+template <typename R, int NPE, bool ONE, bool PI, int MINB> int plan_steps_minb(dnl_engine *h)
 {
-  using L = StepsLayout<R, NPE>;
-  auto *k = k_steps<R, NPE, MINB, ONE>;
+  using L = StepsLayout<R, NPE, PI>;
+  auto *k = k_steps<R, NPE, MINB, ONE, PI>;
   int perSM = 0;
   const size_t smem = L::ROW_BYTES + L::STATE_BYTES;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
@@ -659,15 +659,19 @@ template <typename R, int NPE, bool ONE, int MINB> int plan_steps_minb(dnl_engin
 }
 // FP64: 255 and 168 registers a thread, FP32: 168 and 128 (no spill, a little)
 template <typename R> constexpr int STEPS_BUDGETS[2] = {sizeof(R) == 4 ? 3 : 2, sizeof(R) == 4 ? 4 : 3};
+template <typename R, int NPE, bool ONE, bool PI> int plan_steps_p(dnl_engine *h)
+{
+  const int m = plan_steps_minb<R, NPE, ONE, PI, STEPS_BUDGETS<R>[0]>(h);
+  return m ? m : plan_steps_minb<R, NPE, ONE, PI, STEPS_BUDGETS<R>[1]>(h);
+}
 template <typename R, int NPE, bool ONE> int plan_steps_t(dnl_engine *h)
 {
-  const int m = plan_steps_minb<R, NPE, ONE, STEPS_BUDGETS<R>[0]>(h);
-  return m ? m : plan_steps_minb<R, NPE, ONE, STEPS_BUDGETS<R>[1]>(h);
+  return h->powerIteration ? plan_steps_p<R, NPE, ONE, true>(h) : plan_steps_p<R, NPE, ONE, false>(h);
 }
 
-template <typename R, int NPE, bool ONE> int launch_steps_t(dnl_engine *h, const StepsArgs &a)
+template <typename R, int NPE, bool ONE, bool PI> int launch_steps_p(dnl_engine *h, const StepsArgs &a)
 {
-  using L = StepsLayout<R, NPE>;
+  using L = StepsLayout<R, NPE, PI>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -679,10 +683,14 @@ template <typename R, int NPE, bool ONE> int launch_steps_t(dnl_engine *h, const
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (h->stepsMinb == STEPS_BUDGETS<R>[0])
-    CK(cudaLaunchKernelEx(&cfg, k_steps<R, NPE, STEPS_BUDGETS<R>[0], ONE>, h->M, a));
+    CK(cudaLaunchKernelEx(&cfg, k_steps<R, NPE, STEPS_BUDGETS<R>[0], ONE, PI>, h->M, a));
   else
-    CK(cudaLaunchKernelEx(&cfg, k_steps<R, NPE, STEPS_BUDGETS<R>[1], ONE>, h->M, a));
+    CK(cudaLaunchKernelEx(&cfg, k_steps<R, NPE, STEPS_BUDGETS<R>[1], ONE, PI>, h->M, a));
   return DNL_OK;
+}
+template <typename R, int NPE, bool ONE> int launch_steps_t(dnl_engine *h, const StepsArgs &a)
+{
+  return h->powerIteration ? launch_steps_p<R, NPE, ONE, true>(h, a) : launch_steps_p<R, NPE, ONE, false>(h, a);
 }
 
 // calls f<R, NPE, ONE>(args...) for the engine's precision, element and materials
@@ -693,8 +701,7 @@ template <typename R, int NPE, bool ONE> int launch_steps_t(dnl_engine *h, const
        : (h->npe == 8 ? (h->oneMat ? f<double, 8, true>(__VA_ARGS__) : f<double, 8, false>(__VA_ARGS__))          \
                       : (h->oneMat ? f<double, 4, true>(__VA_ARGS__) : f<double, 4, false>(__VA_ARGS__))))
 
-// Whether runs of this engine go through k_steps: a single model with the
-// Courant time step whose tiles all fit on the GPU at once at one of the
+// Whether runs of this engine go through k_steps: a single model whose tiles all fit on the GPU at once at one of the
 // register budgets (FP64: 444 tiles, 7,104 hexahedra; FP32: 592 tiles, 9,472
 // hexahedra).  At the largest sizes the gain over graph replays is 4 to 8 %,
 // at a few tiles a third; with more blocks per SM the element phase spills
@@ -703,7 +710,7 @@ void plan_steps(dnl_engine *h)
 {
   h->stepsMinb = 0;
   int coop = 0;
-  if (h->nInst != 1 || h->powerIteration ||
+  if (h->nInst != 1 ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device) != cudaSuccess || !coop)
     return;
   h->stepsMinb = DNL_STEPS_DISPATCH(plan_steps_t, h);
@@ -718,6 +725,7 @@ int launch_steps(dnl_engine *h, int n, bool timed)
   a.nIncs = n;
   a.bar = h->stepsBar;
   a.err = h->derr;
+  a.pimax = h->stepsPhase + 4;
   a.phase = timed ? h->stepsPhase : nullptr;
   if (h->histOn)
   {
@@ -729,7 +737,7 @@ int launch_steps(dnl_engine *h, int n, bool timed)
     a.nValues = (int)h->nValues;
     a.kin = h->itemsKinetic;
   }
-  CK(cudaMemsetAsync(h->stepsBar, 0, sizeof(unsigned), h->stream));
+  CK(cudaMemsetAsync(h->stepsBar, 0, 4 * sizeof(unsigned long long), h->stream)); // and the maxima
   int rc = DNL_STEPS_DISPATCH(launch_steps_t, h, a);
   h->launches++;
   return rc;
@@ -1039,7 +1047,7 @@ int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_e
                // zeroed at creation, from here to o_ip
                o_energy = reserve(sizeof(double) * (3 + ENERGY_PARTS) * nI), o_err = reserve(sizeof(int)),
                o_stats = reserve(sizeof(unsigned long long) * 5), o_done = reserve(sizeof(unsigned) * 2),
-               o_steps = reserve(sizeof(unsigned long long) * 4),
+               o_steps = reserve(sizeof(unsigned long long) * 7),
                o_act = reserve(sizeof(int)), o_actlist = reserve(sizeof(int) * nI),
                o_acttile = reserve(sizeof(int) * (nI + 1)), o_actnode = reserve(sizeof(int) * (nI + 1)),
                o_actelem = reserve(sizeof(int) * (nI + 1)), o_due = reserve(sizeof(int)),
@@ -1100,7 +1108,7 @@ int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_e
   M.done_count = (unsigned *)(A + o_done);
   M.step_due = M.done_count + 1;
   h->stepsPhase = (unsigned long long *)(A + o_steps);
-  h->stepsBar = (unsigned *)(h->stepsPhase + 3);
+  h->stepsBar = (unsigned *)(h->stepsPhase + 3); // then the power iteration's three maxima
   M.act_count = (int *)(A + o_act);
   M.act_list = (int *)(A + o_actlist);
   M.act_tile_pre = (int *)(A + o_acttile);

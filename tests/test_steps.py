@@ -93,3 +93,30 @@ def test_steps_stop_at_a_failed_element_and_keep_timings():
         t = e.timings()
         assert min(t.values()) > 0.0
         assert t["element_ms"] + t["nodal_ms"] + t["timestep_ms"] <= t["run_ms"]
+
+
+@pytest.mark.parametrize("precision", [_abi.PREC_FP64, _abi.PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("name", ["axi", "hex-17", "hex-speed", "plane", "bar-297-tiles"])
+def test_power_iteration_in_steps(name, precision):
+    """The power-iteration time step inside the launch: same increments, and
+    time steps, iteration by iteration the sums of its own kernel; a run cut
+    into pieces goes on from the kept vector."""
+    d = MODELS[name](precision).copy(ts_method=_abi.TS_POWER_ITERATION, ts_freq=2)
+    out = []
+    for forced, pieces in ((True, [24]), (False, [24]), (False, [1, 6, 17])):
+        with engine(d) as e:
+            e.init()
+            if forced:
+                e.set_variant(0)
+            for n in pieces:
+                e.run(max_incs=n)
+            c = e.control()
+            out.append((e.nodes(_abi.NODE_COORDS), e.ips(), c["increment"], c["time"], c["time_step"], c["status"]))
+    ref, one, cut = out
+    assert ref[2] == one[2] == cut[2] and ref[5] == one[5] == cut[5] == 0
+    assert np.array_equal(one[0], cut[0]) and np.array_equal(one[1], cut[1]) and one[3:5] == cut[3:5]
+    assert abs(one[4] - ref[4]) <= 1e-11 * ref[4]
+    # the time steps differ by rounding at most, so the states do as two FP64 or
+    # two mixed runs a rounding apart
+    assert helpers.rel_err(one[0], ref[0]) < (1e-12 if precision == _abi.PREC_FP64 else 1e-7)
+    assert helpers.field_errors(one[1], ref[1]).max() < (1e-8 if precision == _abi.PREC_FP64 else 1e-3)
