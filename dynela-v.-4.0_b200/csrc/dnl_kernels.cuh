@@ -62,6 +62,16 @@ __device__ __forceinline__ void pdl_wait()
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A node vector (32 bytes) in one 256-bit load: the element pass gathers two
+// per point, as 16 + 8 bytes each 84.0 us per increment on the 153,600-element
+// bar (mixed), so 83.1.  Not for vectors that the same kernel writes.
+__device__ __forceinline__ double4 ld_vec(const double4 *p)
+{
+  double4 v;
+  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+
 template <typename R> struct V4;
 template <> struct V4<double> { using type = double4; };
 template <> struct V4<float> { using type = float4; };
@@ -759,8 +769,8 @@ template <typename R, bool ONE = false> struct EngineIo
   using R4 = typename V4<R>::type;
   const DevModel &M;
   int q, f0;
-  __device__ __forceinline__ double4 x(int n) const { return M.x[n]; }
-  __device__ __forceinline__ double4 u(int n) const { return M.u[f0][n]; }
+  __device__ __forceinline__ double4 x(int n) const { return ld_vec(M.x + n); }
+  __device__ __forceinline__ double4 u(int n) const { return ld_vec(M.u[f0] + n); }
   __device__ __forceinline__ const MatDev &mat(int e) const { return M.mat[M.emat[e]]; }
   __device__ __forceinline__ const MatDev *matp(int e) const { return M.mat + M.emat[e]; }
   __device__ __forceinline__ JC<R, ONE> law(int e) const
@@ -1948,6 +1958,47 @@ __global__ void __launch_bounds__(TILE, 4) k_element_mode(DevModel M, int nTiles
 // at full occupancy, which is what hides the latency of its gather.  The
 // component's force is still summed over the node's slots in element order.
 constexpr int NODAL_THREADS = 128;
+__device__ __forceinline__ void put_component(double4 *v, int c, double val)
+{
+  if (c == 2)
+    reinterpret_cast<double2 *>(v)[1] = make_double2(val, 0.0);
+  else
+    reinterpret_cast<double *>(v)[c] = val;
+}
+// Boundary condition of component c: its values after the increment, and those
+// of field f0 of before it (both fields are written).
+__device__ __forceinline__ void nodal_bc(const DevModel &M, int i, int c, unsigned code, int f0, double t, double dt,
+                                         double &du, double &v1, double &a1)
+{
+  if (code == DNL_BC_RESTRAIN)
+  {
+    // BoundaryRestrain.C:98-128
+    du = v1 = a1 = 0.0;
+    put_component(M.u[f0] + i, c, 0.0);
+    put_component(M.v[f0] + i, c, 0.0);
+    put_component(M.a[f0] + i, c, 0.0);
+  }
+  else
+  {
+    // BoundarySpeed.C:139-206
+    const double sv = reinterpret_cast<const double *>(M.bcval + i)[c];
+    const int fn = reinterpret_cast<const int *>(M.bcfun + i)[c];
+    double va = sv, vb = sv, acc = 0.0;
+    if (fn >= 0)
+    {
+      const double fa = func_value(M, fn, t), fb = func_value(M, fn, t + dt);
+      acc = (fb - fa) * sv / dt;
+      va = fa * sv;
+      vb = fb * sv;
+    }
+    a1 = acc;
+    v1 = vb;
+    du = vb * dt;
+    put_component(M.u[f0] + i, c, va * dt);
+    put_component(M.v[f0] + i, c, va);
+    put_component(M.a[f0] + i, c, acc);
+  }
+}
 template <typename R, int DIM>
 __device__ __forceinline__ void nodal_update(const DevModel &M, int i, int c, const Ctl *C)
 {
@@ -2003,45 +2054,105 @@ __device__ __forceinline__ void nodal_update(const DevModel &M, int i, int c, co
   // the z thread also writes the (zero) fourth word, so that every 32-byte
   // sector of the node vectors is written whole (a partly written sector
   // costs a read of it from DRAM when it leaves the L2)
-  auto put = [&](double4 *v, double val) {
-    if (c == 2)
-      reinterpret_cast<double2 *>(v)[1] = make_double2(val, 0.0);
-    else
-      reinterpret_cast<double *>(v)[c] = val;
-  };
-  if (code == DNL_BC_RESTRAIN)
-  {
-    // BoundaryRestrain.C:98-128 (both fields)
-    du = v1 = a1 = 0.0;
-    put(M.u[f0] + i, 0.0);
-    put(M.v[f0] + i, 0.0);
-    put(M.a[f0] + i, 0.0);
-  }
-  else if (code == DNL_BC_SPEED)
-  {
-    // BoundarySpeed.C:139-206 (both fields)
-    const double sv = reinterpret_cast<const double *>(M.bcval + i)[c];
-    const int fn = reinterpret_cast<const int *>(M.bcfun + i)[c];
-    double va = sv, vb = sv, acc = 0.0;
-    if (fn >= 0)
-    {
-      const double fa = func_value(M, fn, t), fb = func_value(M, fn, t + dt);
-      acc = (fb - fa) * sv / dt;
-      va = fa * sv;
-      vb = fb * sv;
-    }
-    a1 = acc;
-    v1 = vb;
-    du = vb * dt;
-    put(M.u[f0] + i, va * dt);
-    put(M.v[f0] + i, va);
-    put(M.a[f0] + i, acc);
-  }
+  auto put = [&](double4 *v, double val) { put_component(v, c, val); };
+  if (code == DNL_BC_RESTRAIN || code == DNL_BC_SPEED)
+    nodal_bc(M, i, c, code, f0, t, dt, du, v1, a1);
   put(M.x + i, X + du);
   put(M.disp + i, D + du);
   put(M.u[f1] + i, du);
   put(M.v[f1] + i, v1);
   put(M.a[f1] + i, a1);
+}
+
+// ld_vec in a kernel that writes node vectors: stays where it is
+__device__ __forceinline__ double4 ld32(const double4 *p)
+{
+  double4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p) : "memory");
+  return v;
+}
+// a node vector in one 256-bit store
+__device__ __forceinline__ void st32(double4 *p, double x, double y, double z)
+{
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(0.0) : "memory");
+}
+// two force slots (FP32) in one access
+__device__ __forceinline__ void ld_slots(const float4 *p, float4 &a, float4 &b)
+{
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+               : "l"(p));
+}
+__device__ __forceinline__ void ld_slots(const double4 *p, double4 &a, double4 &b)
+{
+  a = ld32(p);
+  b = ld32(p + 1);
+}
+
+// The update of one node (nodal_update of its three components, the same
+// arithmetic): every node vector and every pair of slots is one 32-byte access.
+template <typename R, int DIM> __device__ __forceinline__ void nodal_update_node(const DevModel &M, int i, const Ctl *C)
+{
+  using R4 = typename V4<R>::type;
+  constexpr int W = DIM == 3 ? 8 : 4;
+  const double m = M.mass[i];
+  const unsigned codes = M.bc[i];
+  const double4 X = ld32(M.x + i), D = ld32(M.disp + i);
+  if (!C->active)
+    return;
+  const int f0 = C->f0, f1 = 1 - f0;
+  const double4 V = ld32(M.v[f0] + i), A = ld32(M.a[f0] + i);
+  double f[3] = {0.0, 0.0, 0.0};
+  if (M.slotW == W)
+  {
+    R4 s[W];
+    const R4 *p = reinterpret_cast<const R4 *>(M.slot) + (size_t)W * i;
+#pragma unroll
+    for (int j = 0; j < W; j += 2)
+      ld_slots(p + j, s[j], s[j + 1]);
+#pragma unroll
+    for (int j = 0; j < W; j++)
+    {
+      f[0] += (double)s[j].x;
+      f[1] += (double)s[j].y;
+      f[2] += (double)s[j].z;
+    }
+  }
+  else
+    for (int k = M.csr_off[i]; k < M.csr_off[i + 1]; k++)
+    {
+      const R4 s = reinterpret_cast<const R4 *>(M.slot)[k];
+      f[0] += (double)s.x;
+      f[1] += (double)s.y;
+      f[2] += (double)s.z;
+    }
+  const double dt = C->dt_eff, t = C->t;
+  const double beta = C->beta, gam = C->gammaN, alphaM = C->alphaM;
+  const double v0[3] = {V.x, V.y, V.z}, a0[3] = {A.x, A.y, A.z};
+  double du[3], v1[3], a1[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+  {
+    du[c] = dt * (v0[c] + (0.5 - beta) * dt * a0[c]);
+    v1[c] = v0[c] + (1.0 - gam) * dt * a0[c];
+    a1[c] = (c < DIM) ? f[c] / m : 0.0;
+    a1[c] = (a1[c] - alphaM * a0[c]) / (1.0 - alphaM);
+    v1[c] += gam * dt * a1[c];
+    du[c] += beta * (dt * dt) * a1[c];
+  }
+  if (codes)
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+    {
+      const unsigned code = (codes >> (2 * c)) & 3u;
+      if (code == DNL_BC_RESTRAIN || code == DNL_BC_SPEED)
+        nodal_bc(M, i, c, code, f0, t, dt, du[c], v1[c], a1[c]);
+    }
+  st32(M.x + i, X.x + du[0], X.y + du[1], X.z + du[2]);
+  st32(M.disp + i, D.x + du[0], D.y + du[1], D.z + du[2]);
+  st32(M.u[f1] + i, du[0], du[1], du[2]);
+  st32(M.v[f1] + i, v1[0], v1[1], v1[2]);
+  st32(M.a[f1] + i, a1[0], a1[1], a1[2]);
 }
 
 // A single model: one thread per (node, component).
@@ -2057,22 +2168,24 @@ __global__ void __launch_bounds__(NODAL_THREADS) k_nodal(DevModel M)
     nodal_update<R, DIM>(M, i, c, M.ctl);
 }
 
-// A batch: a grid-stride loop over the (node, component) pairs of the running
-// instances only (k_active_list), so that stopped instances cost nothing.
+// A batch: a grid-stride loop over the nodes of the running instances only
+// (k_active_list), so that stopped instances cost nothing.  One thread per
+// node, as each finds its instance by a search: on 24 bars (549,000 hexahedra)
+// 57 us per increment with one per component, 50 so.  A single model has no
+// search, and a thread per node is slower there on 22,000 nodes (17.3 -> 18.4 us
+// per increment), faster on 158,000 (84.0 -> 83.0) and the same on 538,000.
 template <typename R, int DIM>
 __global__ void __launch_bounds__(NODAL_THREADS) k_nodal_batch(DevModel M)
 {
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k == 0)
     *M.step_due = 1u;
-  const int na = *M.act_count;
-  const long long n3 = 3LL * M.act_node_pre[na];
-  for (long long kk = k; kk < n3; kk += (long long)gridDim.x * blockDim.x)
+  const int na = *M.act_count, n = M.act_node_pre[na];
+  for (int j = k; j < n; j += gridDim.x * blockDim.x)
   {
-    const int j = (int)(kk / 3), c = (int)(kk - 3LL * j);
     const int a = find_segment(M.act_node_pre, na, j);
     const Ctl *C = M.ctl + M.act_list[a];
-    nodal_update<R, DIM>(M, C->node_begin + (j - M.act_node_pre[a]), c, C);
+    nodal_update_node<R, DIM>(M, C->node_begin + (j - M.act_node_pre[a]), C);
   }
 }
 
@@ -2287,6 +2400,36 @@ __device__ __forceinline__ double charlen_q4(const double3 P[4])
   return (x31 * y42 + x24 * y31) / sqrt(2.0 * (x24 * x24 + y42 * y42 + x31 * x31 + y31 * y31));
 }
 
+// NPE values of component run `comp` of element e's points, as 16-byte loads
+// (an element's points are NPE consecutive values of a run).
+template <typename R, int NPE>
+__device__ __forceinline__ void element_values(const DevModel &M, int comp, int e, R (&v)[NPE])
+{
+  const R *p = reinterpret_cast<const R *>(M.ip) + ip_index(comp, e * NPE);
+  if constexpr (sizeof(R) == 4)
+  {
+#pragma unroll
+    for (int k = 0; k < NPE / 4; k++)
+    {
+      const float4 a = reinterpret_cast<const float4 *>(p)[k];
+      v[4 * k] = a.x;
+      v[4 * k + 1] = a.y;
+      v[4 * k + 2] = a.z;
+      v[4 * k + 3] = a.w;
+    }
+  }
+  else
+  {
+#pragma unroll
+    for (int k = 0; k < NPE / 2; k++)
+    {
+      const double2 a = reinterpret_cast<const double2 *>(p)[k];
+      v[2 * k] = a.x;
+      v[2 * k + 1] = a.y;
+    }
+  }
+}
+
 // Model::computeCourantTimeStep (Model.C:636-669): min over elements of l_e/c_e
 // with the elongation wave speed of the mean point density (Element.C:343-359).
 // One thread per element, a segmented warp-shuffle min over the lanes of one
@@ -2297,10 +2440,22 @@ __device__ __forceinline__ void courant_warp(const DevModel &M, int e, int lane,
   double ratio = 1e300;
   if (act)
   {
+    int node[NPE];
+#pragma unroll
+    for (int k = 0; k < NPE / 4; k++)
+    {
+      const int4 c4 = reinterpret_cast<const int4 *>(M.conn + (size_t)e * NPE)[k];
+      node[4 * k] = c4.x;
+      node[4 * k + 1] = c4.y;
+      node[4 * k + 2] = c4.z;
+      node[4 * k + 3] = c4.w;
+    }
     double3 P[NPE];
 #pragma unroll
     for (int n = 0; n < NPE; n++)
-      P[n] = d3(M.x[M.conn[e * NPE + n]]);
+      P[n] = d3(ld32(M.x + node[n]));
+    R dens[NPE]; // before the geometry, so that it arrives meanwhile
+    element_values<R, NPE>(M, DNL_IP_DENSITY, e, dens);
     double len;
     if constexpr (NPE == 8)
       len = charlen_hex(P);
@@ -2309,7 +2464,7 @@ __device__ __forceinline__ void courant_warp(const DevModel &M, int e, int lane,
     double rho = 0.0;
 #pragma unroll
     for (int g = 0; g < NPE; g++)
-      rho += (double)ipv<R>(M, DNL_IP_DENSITY, e * NPE + g);
+      rho += (double)dens[g];
     rho /= NPE;
     const MatDev &mp = M.mat[M.emat[e]];
     ratio = len / sqrt(mp.wave2 / rho);
@@ -2914,36 +3069,6 @@ template <int NPE> __device__ __forceinline__ double extrapolation_weight(int n,
     return m == 3 ? (5.0 + 3.0 * r3) / 4 : m == 2 ? (-1.0 - r3) / 4 : m == 1 ? (-1.0 + r3) / 4 : (5.0 - 3.0 * r3) / 4;
   else
     return m == 2 ? 1.0 + r3 / 2 : m == 1 ? -0.5 : 1.0 - r3 / 2;
-}
-
-// NPE values of component run `comp` of element e's points, as 16-byte loads
-// (an element's points are NPE consecutive values of a run).
-template <typename R, int NPE>
-__device__ __forceinline__ void element_values(const DevModel &M, int comp, int e, R (&v)[NPE])
-{
-  const R *p = reinterpret_cast<const R *>(M.ip) + ip_index(comp, e * NPE);
-  if constexpr (sizeof(R) == 4)
-  {
-#pragma unroll
-    for (int k = 0; k < NPE / 4; k++)
-    {
-      const float4 a = reinterpret_cast<const float4 *>(p)[k];
-      v[4 * k] = a.x;
-      v[4 * k + 1] = a.y;
-      v[4 * k + 2] = a.z;
-      v[4 * k + 3] = a.w;
-    }
-  }
-  else
-  {
-#pragma unroll
-    for (int k = 0; k < NPE / 2; k++)
-    {
-      const double2 a = reinterpret_cast<const double2 *>(p)[k];
-      v[2 * k] = a.x;
-      v[2 * k + 1] = a.y;
-    }
-  }
 }
 
 // Nodal values of point-state quantities as the reference extracts them for

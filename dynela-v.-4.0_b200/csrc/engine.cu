@@ -479,8 +479,8 @@ int launch_nodal(dnl_engine *h)
   const int threads = NODAL_THREADS;
   if (h->nInst > 1)
   {
-    // a batch loops over its running instances' (node, component) pairs
-    const int blocks = (int)std::min<long long>((3LL * h->nN + threads - 1) / threads, 16LL * h->numSMs);
+    // a batch loops over its running instances' nodes
+    const int blocks = std::min((h->nN + threads - 1) / threads, 16 * h->numSMs);
     if (h->precision == DNL_PREC_MIXED)
     {
       if (h->dim == 3)
