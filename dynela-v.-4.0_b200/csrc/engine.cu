@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "dnl_kernels.cuh"
+#include "dnl_pool.h"
 #include "dnl_steps.cuh"
 #include "dnlgpu.h"
 
@@ -84,7 +85,7 @@ struct dnl_engine
   int4 *ditems = nullptr;
   long long *ditemOff = nullptr;
   double *dvalues = nullptr, *dkin = nullptr;
-  double *hvalues = nullptr; // pinned
+  void *itemMem = nullptr; // their allocation
   // read-back staging on the device, kept from call to call (grown on demand)
   void *dstage = nullptr;
   size_t stageBytes = 0;
@@ -130,9 +131,9 @@ template <typename T> int dalloc(dnl_engine *h, T **p, size_t n)
   *p = nullptr;
   if (n == 0)
     n = 1;
-  cudaError_t e = cudaMalloc((void **)p, n * sizeof(T));
+  cudaError_t e = dnl_pool_alloc((void **)p, n * sizeof(T), h->stream);
   if (e != cudaSuccess)
-    return fail(h, DNL_ERR_CUDA, "cudaMalloc of %zu bytes failed: %s", n * sizeof(T), cudaGetErrorString(e));
+    return fail(h, DNL_ERR_CUDA, "allocation of %zu bytes failed: %s", n * sizeof(T), cudaGetErrorString(e));
   h->allocs.push_back(*p);
   return DNL_OK;
 }
@@ -163,12 +164,11 @@ int staging(dnl_engine *h, size_t bytes, void **out)
   {
     if (h->dstage)
     {
-      CK(cudaStreamSynchronize(h->stream));
-      cudaFree(h->dstage);
+      dnl_pool_free(h->dstage, h->stream);
       h->dstage = nullptr;
       h->stageBytes = 0;
     }
-    CK(cudaMalloc(&h->dstage, bytes));
+    CK(dnl_pool_alloc(&h->dstage, bytes, h->stream));
     h->stageBytes = bytes;
   }
   *out = h->dstage;
@@ -1055,11 +1055,11 @@ int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_e
                o_ip = reserve((size_t)DNL_IP_NCOMP * nIPpad * rsz), o_slot = reserve(nSlotCap * 4 * rsz);
   char *A = nullptr;
   {
-    cudaError_t e = cudaMalloc((void **)&A, total);
+    cudaError_t e = dnl_pool_alloc((void **)&A, total, h->stream);
     if (e != cudaSuccess)
     {
       dnl_engine_destroy(h);
-      return fail(nullptr, DNL_ERR_CUDA, "cudaMalloc of %zu bytes failed: %s", total, cudaGetErrorString(e));
+      return fail(nullptr, DNL_ERR_CUDA, "allocation of %zu bytes failed: %s", total, cudaGetErrorString(e));
     }
     h->allocs.push_back(A);
   }
@@ -1331,11 +1331,9 @@ int dnl_engine_destroy(dnl_engine *h)
     cudaStreamSynchronize(h->stream);
   drop_graph(h);
   for (void *p : h->allocs)
-    cudaFree(p);
-  if (h->dstage)
-    cudaFree(h->dstage);
-  if (h->histMem)
-    cudaFree(h->histMem);
+    dnl_pool_free(p, h->stream);
+  dnl_pool_free(h->dstage, h->stream);
+  dnl_pool_free(h->histMem, h->stream);
   free_items(h);
   delete[] h->hctl;
   if (h->stream)
@@ -2053,14 +2051,11 @@ int launch_energies(dnl_engine *h, double *dst, int speed_field, int points)
 
 void free_items(dnl_engine *h)
 {
-  for (void *p : {(void *)h->ditems, (void *)h->ditemOff, (void *)h->dvalues, (void *)h->dkin})
-    if (p)
-      cudaFree(p);
-  if (h->hvalues)
-    cudaFreeHost(h->hvalues);
+  dnl_pool_free(h->itemMem, h->stream);
+  h->itemMem = nullptr;
   h->ditems = nullptr;
   h->ditemOff = nullptr;
-  h->dvalues = h->dkin = h->hvalues = nullptr;
+  h->dvalues = h->dkin = nullptr;
   h->nItems = 0;
   h->nValues = 0;
   h->itemsKinetic = 0;
@@ -2116,11 +2111,15 @@ int dnl_engine_set_items(dnl_engine *h, const dnl_item *items, int32_t n, int64_
   }
   if (n > 0)
   {
-    CK(cudaMalloc((void **)&h->ditems, sizeof(int4) * n));
-    CK(cudaMalloc((void **)&h->ditemOff, sizeof(long long) * n));
-    CK(cudaMalloc((void **)&h->dvalues, sizeof(double) * total));
-    CK(cudaMalloc((void **)&h->dkin, sizeof(double) * 6 * h->nInst));
-    CK(cudaMallocHost((void **)&h->hvalues, sizeof(double) * total));
+    // one allocation: items, offsets, values, kinetic energies
+    char *p = nullptr;
+    CK(dnl_pool_alloc((void **)&p, (sizeof(int4) + sizeof(long long)) * n + sizeof(double) * (total + 6 * h->nInst),
+                      h->stream));
+    h->itemMem = p;
+    h->ditems = (int4 *)p;
+    h->ditemOff = (long long *)(h->ditems + n);
+    h->dvalues = (double *)(h->ditemOff + n);
+    h->dkin = h->dvalues + total;
     CK(cudaMemcpyAsync(h->ditems, it.data(), sizeof(int4) * n, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->ditemOff, off.data(), sizeof(long long) * n, cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
@@ -2156,10 +2155,7 @@ int dnl_engine_gather_items(dnl_engine *h, double *out)
     k_gather_items<double><<<blocks, threads, 0, h->stream>>>(h->M, h->ditems, h->ditemOff, h->nItems, h->dkin,
                                                                  h->dvalues);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(h->hvalues, h->dvalues, sizeof(double) * h->nValues, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
-  memcpy(out, h->hvalues, sizeof(double) * h->nValues);
-  return DNL_OK;
+  return copy(h, out, h->dvalues, sizeof(double) * h->nValues, cudaMemcpyDeviceToHost);
 }
 
 int dnl_engine_set_history(dnl_engine *h, const dnl_history_schedule *sched, int32_t n, int32_t capacity)
@@ -2176,7 +2172,7 @@ int dnl_engine_set_history(dnl_engine *h, const dnl_history_schedule *sched, int
   h->histHost.clear();
   if (h->histMem)
   {
-    cudaFree(h->histMem);
+    dnl_pool_free(h->histMem, h->stream);
     h->histMem = nullptr;
   }
   if (n == 0)
@@ -2186,7 +2182,7 @@ int dnl_engine_set_history(dnl_engine *h, const dnl_history_schedule *sched, int
   // one allocation: count, overflow, last increment, the schedules, the records
   const size_t offLast = 16, offSched = 32, offRec = offSched + ((sizeof(double) * 3 * n + 255) / 256) * 256;
   const size_t bytes = offRec + sizeof(double) * width * cap;
-  CK(cudaMalloc(&h->histMem, bytes));
+  CK(dnl_pool_alloc(&h->histMem, bytes, h->stream));
   char *base = (char *)h->histMem;
   HistRing &H = h->hist;
   H.nSched = n;
@@ -2275,7 +2271,7 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
   for (auto &p : parts)
     total += (p.bytes + 255) / 256 * 256;
   char *save = nullptr;
-  if (cudaMalloc((void **)&save, total) != cudaSuccess)
+  if (dnl_pool_alloc((void **)&save, total, h->stream) != cudaSuccess)
     return fail(h, DNL_ERR_CUDA, "autotune: no room for the state snapshot (%zu bytes)", total);
   size_t off = 0;
   for (auto &p : parts)
@@ -2339,7 +2335,7 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
   for (auto &p : parts)
     CK(cudaMemcpyAsync(const_cast<void *>(p.src), p.dst, p.bytes, cudaMemcpyDeviceToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  cudaFree(save);
+  dnl_pool_free(save, h->stream);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   h->variant = best;

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "dnl_kernels.cuh"
+#include "dnl_pool.h"
 #include "dnlgpu.h"
 
 void dnl_internal_set_error(const char *msg);
@@ -333,15 +334,17 @@ __global__ void __launch_bounds__(TILE) k_mlp_forward(const void *image, const f
 
 struct Work
 {
+  cudaStream_t stream;
   std::vector<void *> allocs;
+  explicit Work(cudaStream_t st) : stream(st) {}
   ~Work()
   {
     for (void *p : allocs)
-      cudaFree(p);
+      dnl_pool_free(p, stream);
   }
   template <typename T> bool alloc(T **p, size_t n)
   {
-    if (cudaMalloc((void **)p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess)
+    if (dnl_pool_alloc((void **)p, n * sizeof(T), stream) != cudaSuccess)
       return false;
     allocs.push_back(*p);
     return true;
@@ -409,11 +412,11 @@ int dnl_mlp_forward(const dnl_mlp *net, const float *d_x, int64_t n, float *d_y,
   if (n == 0)
     return DNL_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  Work w;
+  Work w(st);
   unsigned char *dimg;
   int *derr;
   if (!w.alloc(&dimg, IMAGE_BYTES) || !w.alloc(&derr, 1))
-    return fail_msg(DNL_ERR_CUDA, "dnl_mlp_forward: cudaMalloc failed");
+    return fail_msg(DNL_ERR_CUDA, "dnl_mlp_forward: allocation failed");
   std::vector<unsigned char> img(IMAGE_BYTES);
   build_image(*net, img.data());
   MCK(cudaMemcpyAsync(dimg, img.data(), IMAGE_BYTES, cudaMemcpyHostToDevice, st));
@@ -443,13 +446,13 @@ int dnl_mlp_gradients(const dnl_mlp *net, const float *d_x, const float *d_t, in
   const long long tiles = (n + TILE - 1) / TILE;
   if (tiles > (1 << 20))
     return fail_msg(DNL_ERR_ARG, "dnl_mlp_gradients: too many samples for one call");
-  Work w;
+  Work w(st);
   unsigned char *dimg;
   float *part, *lossp, *dgrad, *dloss;
   int *derr;
   if (!w.alloc(&dimg, IMAGE_BYTES + TRANS_BYTES) || !w.alloc(&part, (size_t)tiles * NPARAM) ||
       !w.alloc(&lossp, tiles) || !w.alloc(&dgrad, NPARAM) || !w.alloc(&dloss, 1) || !w.alloc(&derr, 1))
-    return fail_msg(DNL_ERR_CUDA, "dnl_mlp_gradients: cudaMalloc failed");
+    return fail_msg(DNL_ERR_CUDA, "dnl_mlp_gradients: allocation failed");
   std::vector<unsigned char> img;
   host_train_image(*net, img);
   MCK(cudaMemcpyAsync(dimg, img.data(), img.size(), cudaMemcpyHostToDevice, st));
@@ -481,7 +484,7 @@ int dnl_mlp_train(dnl_mlp *net, const float *d_x, const float *d_t, int64_t n, i
   cudaStream_t st = (cudaStream_t)stream;
   const long long batch = (long long)batch_tiles * TILE;
   const long long steps = (n + batch - 1) / batch;
-  Work w;
+  Work w(st);
   unsigned char *dimg;
   float *part, *lossp, *dw, *dm, *dv, *dstep_loss;
   int *derr, *dperm;
@@ -489,7 +492,7 @@ int dnl_mlp_train(dnl_mlp *net, const float *d_x, const float *d_t, int64_t n, i
       !w.alloc(&lossp, batch_tiles) || !w.alloc(&dw, NPARAM) || !w.alloc(&dm, NPARAM) || !w.alloc(&dv, NPARAM) ||
       !w.alloc(&dstep_loss, (size_t)std::max<long long>(steps * epochs, 1)) || !w.alloc(&derr, 1) ||
       !w.alloc(&dperm, n))
-    return fail_msg(DNL_ERR_CUDA, "dnl_mlp_train: cudaMalloc failed");
+    return fail_msg(DNL_ERR_CUDA, "dnl_mlp_train: allocation failed");
   std::vector<unsigned char> img;
   host_train_image(*net, img);
   MCK(cudaMemcpyAsync(dimg, img.data(), img.size(), cudaMemcpyHostToDevice, st));
