@@ -54,9 +54,9 @@ static constexpr unsigned long long INF_BITS = 0x7ff0000000000000ull;
 // Programmatic dependent launch: the kernels of an increment are launched so
 // that the next one is scheduled as the blocks of the one before leave; each
 // waits here, before its first memory access, until the previous grid has
-// completed and its writes are visible (a no-op after a normal launch).  No
-// kernel triggers its dependents early: blocks of the next kernel holding
-// registers while the previous one still runs slowed the increment.
+// completed and its writes are visible (a no-op after a normal launch).  Only
+// the small Courant kernel triggers its dependents early: blocks of the next
+// kernel holding registers while a large one still runs slowed the increment.
 __device__ __forceinline__ void pdl_wait()
 {
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -806,12 +806,14 @@ template <typename R> struct GlobalState
 {
   const DevModel &M;
   int q;
+  __device__ __forceinline__ bool ready() const { return true; }
   __device__ __forceinline__ R operator()(int c) const { return ipv<R>(M, c, q); }
 };
 template <typename R> struct SharedTile
 {
   const R *buf;
   int t;
+  __device__ __forceinline__ bool ready() const { return true; }
   // a staged tile holds the first DNL_IP_NREAD runs (the pass never reads the others)
   __device__ __forceinline__ R operator()(int c) const { return buf[ip_slot(c) * TILE + t]; }
 };
@@ -943,6 +945,8 @@ __device__ __forceinline__ void element_update(const Io &io, const Ctl *C, Ctl *
   // element-mean volumetric increment (Element::computePressure, Element.C:1125-1143)
   const R trSum = group_sum<NPE>(amask, dE[0] + dE[3] + dE[5]);
 
+  if (!old.ready()) // the old point state, where it is still on its way
+    return;
   // total strain: Strain += dE, then the final rotation (Element.C:1116-1161)
   {
     R strain[6];
@@ -1426,19 +1430,21 @@ template <typename R, int NPE, int MINB, int PTS = TILE, bool ONE = false>
 __global__ void __launch_bounds__(PTS, MINB) k_element(DevModel M, int nTiles)
 {
   static_assert(PTS == TILE || PTS == 2 * TILE || 2 * PTS == TILE, "PTS: half, one or two tiles");
-  pdl_wait();
   constexpr int ROW = ElemShape<NPE>::template pass_row<R>;
   __shared__ __align__(16) R sh[PTS * ROW];
   const int lane = threadIdx.x & 31;
   const int g = lane & (NPE - 1);
   const int base = lane & ~(NPE - 1);
   const TileMap<NPE> map{M, nTiles};
+  const int t = PTS >= TILE ? (int)(threadIdx.x % TILE) : (int)((blockIdx.x % 2) * PTS + threadIdx.x);
   const int slot = PTS >= TILE ? (int)(blockIdx.x * (PTS / TILE) + threadIdx.x / TILE) : (int)(blockIdx.x / 2);
+  // a single model's connectivity, which nobody writes, before the wait
+  int node = M.nInst == 1 && slot < nTiles ? M.conn[slot * TILE + t] : 0;
+  pdl_wait();
   if (slot >= map.count())
     return;
   int tile, inst;
   map.get(slot, tile, inst);
-  const int t = PTS >= TILE ? (int)(threadIdx.x % TILE) : (int)((blockIdx.x % 2) * PTS + threadIdx.x);
   const int q = tile * TILE + t;
   const int e = q / NPE;
   Ctl *C = M.ctl + inst;
@@ -1446,9 +1452,11 @@ __global__ void __launch_bounds__(PTS, MINB) k_element(DevModel M, int nTiles)
   const unsigned amask = __ballot_sync(0xffffffffu, act);
   if (!act)
     return;
+  if (M.nInst > 1)
+    node = M.conn[q];
   GlobalState<R> old{M, q};
   EngineIo<R, ONE> io{M, q, C->f0};
-  element_update<R, NPE>(io, C, C, q, e, g, base, amask, M.conn[q], old, sh + threadIdx.x * ROW,
+  element_update<R, NPE>(io, C, C, q, e, g, base, amask, node, old, sh + threadIdx.x * ROW,
                          sh + (threadIdx.x - g) * ROW);
 }
 
@@ -1583,6 +1591,94 @@ __global__ void __launch_bounds__(TILE, MINB) k_element_tma(DevModel M, int nTil
       element_update<R, NPE>(io, C, C, q, e, g, base, amask, conn[b][t], old, rows + t * ROW, rows + (t - g) * ROW);
     }
     __syncthreads(); // the buffer is refilled two tiles later
+  }
+}
+
+// The old point state of a tile on its way into shared memory: ready() waits
+// for the bulk copy (bounded; false, with the error flag set, when it gave up).
+template <typename R> struct ArrivingTile
+{
+  const R *buf;
+  int t;
+  uint64_t *bar;
+  uint32_t phase;
+  int *err;
+  __device__ __forceinline__ bool ready() const
+  {
+    if (mbar_wait(bar, phase))
+      return true;
+    atomicExch(err, 1);
+    mbar_wait(bar, phase); // no thread leaves while the copy into the block's memory is in flight
+    return false;
+  }
+  __device__ __forceinline__ R operator()(int c) const { return buf[ip_slot(c) * TILE + t]; }
+};
+
+// Element pass, a tile's point state by one bulk copy issued before anything
+// else, so that the state arrives while the nodes are gathered and the strain
+// increment forms: the loads of k_element come one group after the other, as
+// its registers allow (at 80 registers a thread, 24 warps an SM, each warp waits
+// for memory half a dozen times).  Whole increments, 80 registers, k_element ->
+// this: 153,600 hexahedra 91.9 -> 78.9 us, plate of 491,520 291 -> 263 (the
+// staged pass with 4 blocks an SM 274); batches, staged -> this: 24 bars (543,000
+// hexahedra) 346 -> 346, 120 smaller ones (858,000) 590 -> 561, 8 small ones 34.3
+// -> 31.8, four running of 200 34.7 -> 36.  LOOP false: a block per work slot
+// (TileMap) of a single model.  LOOP true: batches, the blocks walk over the
+// slots of the running instances, ONCE_BLOCKS blocks per resident one, so that
+// they still come and go (blocks that all stay in step are slower: the staged
+// kernels) and a batch of which few instances run does not start a block for
+// every tile.
+constexpr int ONCE_BLOCKS = 16;
+template <typename R, int NPE, int MINB, bool ONE, bool LOOP>
+__global__ void __launch_bounds__(TILE, MINB) k_element_once(DevModel M, int nTiles, int *err)
+{
+  constexpr int ROW = ElemShape<NPE>::template pass_row<R>;
+  constexpr uint32_t STATE_BYTES = DNL_IP_NREAD * TILE * sizeof(R);
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  R *state = reinterpret_cast<R *>(smem_raw), *rows = reinterpret_cast<R *>(smem_raw + STATE_BYTES);
+  __shared__ __align__(8) uint64_t bar;
+  const int t = threadIdx.x;
+  if (t == 0)
+  {
+    mbar_init(&bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  int node = LOOP ? 0 : M.conn[blockIdx.x * TILE + t]; // nobody writes it
+  pdl_wait();
+  const TileMap<NPE> map{M, nTiles};
+  const int nSlots = map.count();
+  uint32_t phase = 0;
+  for (int slot = blockIdx.x; slot < nSlots; slot += gridDim.x, phase ^= 1)
+  {
+    int tile, inst;
+    map.get(slot, tile, inst);
+    if (t == 0)
+    {
+      if (LOOP)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_expect_tx(&bar, STATE_BYTES);
+      bulk_g2s_ef(state, reinterpret_cast<const R *>(M.ip) + (size_t)tile * DNL_IP_NCOMP * TILE, STATE_BYTES, &bar);
+    }
+    if (!LOOP || slot == (int)blockIdx.x)
+      __syncthreads(); // the barrier is set up for all who wait on it
+    const int g = t & (NPE - 1), base = t & 31 & ~(NPE - 1);
+    const int q = tile * TILE + t, e = q / NPE;
+    Ctl *C = M.ctl + inst;
+    const bool act = e >= C->elem_begin && e < C->elem_end && C->active;
+    const unsigned amask = __ballot_sync(0xffffffffu, act);
+    ArrivingTile<R> old{state, t, &bar, phase, err};
+    if (act)
+    {
+      if (LOOP)
+        node = M.conn[q];
+      EngineIo<R, ONE> io{M, q, C->f0};
+      element_update<R, NPE>(io, C, C, q, e, g, base, amask, node, old, rows + t * ROW, rows + (t - g) * ROW);
+    }
+    else
+      old.ready(); // see there
+    if (!LOOP)
+      return;
+    __syncthreads(); // the tile has been read
   }
 }
 
@@ -2512,6 +2608,10 @@ __global__ void __launch_bounds__(256) k_courant_finish(DevModel M)
   const int nE32 = (M.nE + 31) & ~31; // whole warps, so every lane takes the same trips
   // read from the flag the nodal pass wrote, not from the control block, which
   // the block that finishes the increment rewrites while others may still read
+  // the next increment's first blocks come while this small grid still runs (the
+  // element pass reads its connectivity meanwhile): 83.1 -> 82.4 us per increment
+  // on the 153,600-element bar (mixed), 159.4 -> 157.9 (FP64)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (*M.step_due == 0u)
   {
     // a single model whose time step is not due: no minimum to wait for, the

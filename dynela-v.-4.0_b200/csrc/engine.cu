@@ -264,18 +264,18 @@ std::vector<int> node_order_of(const dnl_model_desc *d, int npe)
 struct Variant
 {
   const char *name;
-  int tma;  // 0 plain, 1 bulk-copy state, 2 fully staged
+  int tma;  // 0 plain, 1 bulk-copy state, 2 fully staged, 3 bulk-copy state, a block per tile
   int minb; // blocks per SM of the register budget
   int pts;  // points (threads) per block
 };
-// each precision: two plain budgets, then persistent staged tiles from the most
+// each precision: two plain budgets (FP32: the tile's state by one bulk copy at 80 registers instead of the first), then persistent staged tiles from the most
 // blocks per SM (fewest registers, most spilled) to the fewest (no spills)
 // then the fully staged kernel (node gathers one tile ahead as well)
 // then plain blocks of half a tile (8 hexahedra) and of two tiles (32) at
 // the register budgets of the 128-point ones; in FP32 also the plain passes
 // at 48 registers (plain64/20, plain/10: 40 warps per SM, no more spilled
 // than at 64 registers)
-const Variant kVariantsF32[] = {{"plain/6", 0, 6, 128},     {"plain/8", 0, 8, 128},    {"tma/4", 1, 4, 128},
+const Variant kVariantsF32[] = {{"once/6", 3, 6, 128},     {"plain/8", 0, 8, 128},    {"tma/4", 1, 4, 128},
                                 {"plain64/20", 0, 20, 64},  {"tma/3", 1, 3, 128},      {"stage/4", 2, 4, 128},
                                 {"stage/3", 2, 3, 128},     {"stage/2", 2, 2, 128},    {"plain64/12", 0, 12, 64},
                                 {"plain64/16", 0, 16, 64},  {"plain/10", 0, 10, 128},  {"plain256/4", 0, 4, 256}};
@@ -354,6 +354,31 @@ template <typename R, int NPE, bool ONE, int MINB> int launch_stage(dnl_engine *
   return DNL_OK;
 }
 
+template <typename R, int NPE, bool ONE, bool LOOP, int MINB> int launch_once_t(dnl_engine *h)
+{
+  const size_t smem = DNL_IP_NREAD * TILE * sizeof(R) + TILE * ElemShape<NPE>::template pass_row<R> * sizeof(R);
+  auto *k = k_element_once<R, NPE, MINB, ONE, LOOP>;
+  static int perSM = -1; // per instantiation
+  if (perSM < 0)
+  {
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, TILE, smem));
+    if (perSM < 1)
+      perSM = 1;
+  }
+  const int slots = h->nTiles + h->nInst - 1; // see launch_plain
+  launch_pdl(h, k, LOOP ? std::min(slots, ONCE_BLOCKS * perSM * h->numSMs) : slots, TILE, smem, h->M, h->nTiles, h->derr);
+  return DNL_OK;
+}
+// (a batch has a material per instance at least)
+template <typename R, int NPE, bool ONE, int MINB> int launch_once(dnl_engine *h)
+{
+  if constexpr (!ONE)
+    if (h->nInst > 1)
+      return launch_once_t<R, NPE, false, true, MINB>(h);
+  return launch_once_t<R, NPE, ONE, false, MINB>(h);
+}
+
 template <int NPE, int MODE> int launch_mode(dnl_engine *h)
 {
   const size_t smem = MODE == MODE_GUESS ? mlp::SMEM_BYTES : 0;
@@ -390,7 +415,7 @@ template <typename R, int NPE, bool ONE> int launch_variant(dnl_engine *h, int v
   {
     switch (v)
     {
-    case 0: return launch_plain<R, NPE, ONE, 6>(h);
+    case 0: return launch_once<R, NPE, ONE, 6>(h);
     case 1: return launch_plain<R, NPE, ONE, 8>(h);
     case 2: return launch_tma<R, NPE, ONE, 4>(h);
     case 3: return launch_plain<R, NPE, ONE, 20, TILE / 2>(h);
@@ -1265,10 +1290,10 @@ int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_e
   M.nSpeed = nSpeed;
   // the layout k_slot_pos chose: npe slots per node when no node has more
   M.slotW = counts[1] <= h->npe ? h->npe : 0;
-  // batches start on a persistent variant: the plain one launches a block per
-  // tile of the whole batch, which the tail of a batch (few instances still
+  // FP64 batches start on a persistent variant: the plain one launches a block
+  // per tile of the whole batch, which the tail of a batch (few instances still
   // running) cannot afford
-  h->variant = (h->nInst > 1) ? 6 : 0;
+  h->variant = h->nInst > 1 && h->precision == DNL_PREC_FP64 ? 6 : 0;
   h->powerIteration = (descs[0]->ts_method == DNL_TS_POWER_ITERATION);
   if (h->powerIteration)
   {
@@ -2321,17 +2346,24 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
       best = v;
     }
   }
-  // the trial increments are the next few; later in an impact more points
-  // yield, and there the variant with the most warps holds up best: the plain
-  // pass on 128-point blocks at 48 registers (10 per SM, 40 warps) for a
-  // single model (3-D bar: 0.0714 ms at the start and 0.0743 after 3,000
-  // increments, against 0.0723 and 0.0741-0.0762 for 64-point blocks at 64
-  // registers), the staged kernel with 4 blocks per SM for a batch (plain
-  // variants are not offered to batches).  The preferred variant is kept
-  // when within 1 % of the fastest trial.
-  const int prefer = h->nInst == 1 ? 10 : 5;
-  if (h->precision == DNL_PREC_MIXED && h->variantMs[prefer] > 0.0 && h->variantMs[prefer] <= 1.01 * bestMs)
-    best = prefer;
+  // Mixed single models: a variant by size when it is within 10 % of the fastest
+  // trial.  The builds of 48 and 64 registers contract a multiply and an add
+  // here and there that the others do not, which changes a last bit at a few
+  // points in 10^5 and, through the halving exits of the return at first yield,
+  // the plastic strain rate of single points by percents some hundred
+  // increments later; a model's results should not depend on which of two
+  // variants a few per cent apart won a trial of microseconds.  Below 16,000
+  // hexahedra the pass of 80 registers (once/6), from there to 180,000 the plain
+  // one of 48, as tuned models of these sizes have run (trials on 39,900 to
+  // 153,600: 3 to 6 % behind once/6), above the fastest, which is once/6 (plate of
+  // 491,520: 206 against 213 for the staged pass and 216 for the plain one).  A
+  // batch is offered variants of one arithmetic only and takes the fastest.
+  if (h->nInst == 1 && h->precision == DNL_PREC_MIXED && h->nE < 180000)
+  {
+    const int prefer = h->nE < 16000 ? 0 : 10;
+    if (h->variantMs[prefer] > 0.0 && h->variantMs[prefer] <= 1.1 * bestMs)
+      best = prefer;
+  }
   for (auto &p : parts)
     CK(cudaMemcpyAsync(const_cast<void *>(p.src), p.dst, p.bytes, cudaMemcpyDeviceToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));

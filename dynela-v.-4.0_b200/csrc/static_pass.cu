@@ -96,6 +96,7 @@ struct PlainState
 {
   const double *ip;
   int nIP, q;
+  __device__ __forceinline__ bool ready() const { return true; }
   __device__ __forceinline__ double operator()(int c) const { return ip[(size_t)c * nIP + q]; }
 };
 

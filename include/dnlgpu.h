@@ -358,17 +358,17 @@ int dnl_engine_set_graph_increments(dnl_engine *h, int32_t n);
 /* Number of kernel launches issued on the device by the last run call. */
 int64_t dnl_engine_launch_count(const dnl_engine *h);
 
-/* Element-pass autotuner (hex8 models): times each kernel variant (staging
- * scheme: plain, bulk-copied point state, or every input staged; register
- * budget; points per block for the plain kernel: 64, 128 or 256, i.e. 8, 16
- * or 32 hexahedra; names from dnl_variant_name) over `steps` increments
- * run from a saved copy of the state, keeps the fastest for the following runs
- * (on the mixed path a preferred variant when it is within 1 % of the fastest,
- * as it holds up best later in an impact: the plain pass on 64-point blocks,
- * 9, for a single model, the staged 4-blocks-per-SM pass, 5, for a batch) and
- * restores the state.  A batch (several instances) is offered the
- * persistent variants only (its ms entries for the plain ones are -1): the
- * plain variants launch a block per tile of the whole batch at every
+/* Element-pass autotuner (hex8 models): times each kernel variant (how the
+ * point state reaches the block: plain loads, one bulk copy per tile, bulk
+ * copies a tile ahead, or every input staged; register budget; points per
+ * block for the plain kernel: 64, 128 or 256, i.e. 8, 16 or 32 hexahedra; names
+ * from dnl_variant_name) over `steps` increments run from a saved copy of the
+ * state, keeps the fastest for the following runs and restores the state.  On
+ * the mixed path a single model of less than 180,000 hexahedra keeps a variant
+ * by its size when that is within 10 % of the fastest (once/6, 0, below 16,000,
+ * plain/10, 10, above), so that its results do not depend on the trial's timing.
+ * A batch (several instances) is not offered the plain variants (their ms
+ * entries are -1): they launch a block per tile of the whole batch at every
  * increment, even when few instances still run.  No counterpart in the
  * reference (its element loop has one implementation). */
 int dnl_engine_autotune(dnl_engine *h, int32_t steps);
