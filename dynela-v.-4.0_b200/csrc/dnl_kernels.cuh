@@ -1622,8 +1622,9 @@ template <typename R> struct ArrivingTile
 // this: 153,600 hexahedra 91.9 -> 78.9 us, plate of 491,520 291 -> 263 (the
 // staged pass with 4 blocks an SM 274); batches, staged -> this: 24 bars (543,000
 // hexahedra) 346 -> 346, 120 smaller ones (858,000) 590 -> 561, 8 small ones 34.3
-// -> 31.8, four running of 200 34.7 -> 36.  LOOP false: a block per work slot
-// (TileMap) of a single model.  LOOP true: batches, the blocks walk over the
+// -> 31.8, four running of 200 34.7 -> 36.  FP64, 128 registers: 153,600
+// hexahedra 157.4 -> 153.5, with two materials 179.7 -> 172.7.  LOOP false: a block per work slot
+// (TileMap) of a single model.  LOOP true (several materials, batches): the blocks walk over the
 // slots of the running instances, ONCE_BLOCKS blocks per resident one, so that
 // they still come and go (blocks that all stay in step are slower: the staged
 // kernels) and a batch of which few instances run does not start a block for
