@@ -18,6 +18,33 @@
 
 namespace dnl
 {
+// A build of k_steps: the kernel, its dynamic shared memory and the blocks per
+// SM of its register budget.  The builds are translation units of their own
+// (steps.cu): the first kernel that a process uses of a unit loads all of the
+// unit's code.  A process's first engine, with all kernels in one unit, with
+// two units of builds apart, with eight: 153,600 hexahedra, which use none of
+// them, 55, 26, 26 ms; 800 quads 44 (two), 34 (eight).
+struct StepsBuild
+{
+  const void *kernel = nullptr;
+  size_t smem = 0;
+  int minb = 0;
+};
+// the fewest blocks (most registers) first
+constexpr int STEPS_BUDGETS = 2;
+template <typename R, int NPE, bool PI> StepsBuild steps_build(bool one, int budget);
+template <> StepsBuild steps_build<float, 4, false>(bool, int);
+template <> StepsBuild steps_build<float, 4, true>(bool, int);
+template <> StepsBuild steps_build<float, 8, false>(bool, int);
+template <> StepsBuild steps_build<float, 8, true>(bool, int);
+template <> StepsBuild steps_build<double, 4, false>(bool, int);
+template <> StepsBuild steps_build<double, 4, true>(bool, int);
+template <> StepsBuild steps_build<double, 8, false>(bool, int);
+template <> StepsBuild steps_build<double, 8, true>(bool, int);
+} // namespace dnl
+
+namespace dnl
+{
 namespace
 {
 
@@ -443,6 +470,19 @@ __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
       for (int k = 0; k < 3; k++)
         A.phase[k] += ns[k];
   }
+}
+
+// A build of k_steps by register budget.
+template <typename R, int NPE, bool ONE, bool PI, int MINB> StepsBuild steps_build_one()
+{
+  using L = StepsLayout<R, NPE, PI>;
+  return {(const void *)k_steps<R, NPE, MINB, ONE, PI>, L::ROW_BYTES + L::STATE_BYTES, MINB};
+}
+template <typename R, int NPE, bool ONE, bool PI> StepsBuild steps_build_budget(int budget)
+{
+  // FP64: 255 and 168 registers a thread, FP32: 168 and 128 (no spill, a little)
+  constexpr int B = sizeof(R) == 4 ? 3 : 2;
+  return budget == 0 ? steps_build_one<R, NPE, ONE, PI, B>() : steps_build_one<R, NPE, ONE, PI, B + 1>();
 }
 
 } // namespace

@@ -67,7 +67,7 @@ struct dnl_engine
   bool forced = false;      // a variant asked for by dnl_engine_set_variant
   // increments in one cooperative launch (dnl_steps.cuh): register budget
   // (blocks per SM), 0 when the model is not run so
-  int stepsMinb = 0;
+  StepsBuild steps;
   unsigned *stepsBar = nullptr;            // grid barrier
   unsigned long long *stepsPhase = nullptr; // [3] phase times (ns)
   double variantMs[DNL_NUM_VARIANTS] = {0};
@@ -668,65 +668,13 @@ int launch_history(dnl_engine *h)
   return DNL_OK;
 }
 
-// Register budgets of k_steps, as blocks per SM: the fewest blocks (most
-// registers) that hold the model's tiles, one per block.
-template <typename R, int NPE, bool ONE, bool PI, int MINB> int plan_steps_minb(dnl_engine *h)
+// The k_steps builds of the engine's precision, element, materials and time step method.
+template <typename R> StepsBuild steps_build_of(const dnl_engine *h, int budget)
 {
-  using L = StepsLayout<R, NPE, PI>;
-  auto *k = k_steps<R, NPE, MINB, ONE, PI>;
-  int perSM = 0;
-  const size_t smem = L::ROW_BYTES + L::STATE_BYTES;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, TILE, smem) != cudaSuccess)
-  {
-    cudaGetLastError();
-    perSM = 0;
-  }
-  return h->nTiles <= perSM * h->numSMs ? MINB : 0;
+  if (h->npe == 8)
+    return h->powerIteration ? steps_build<R, 8, true>(h->oneMat, budget) : steps_build<R, 8, false>(h->oneMat, budget);
+  return h->powerIteration ? steps_build<R, 4, true>(h->oneMat, budget) : steps_build<R, 4, false>(h->oneMat, budget);
 }
-// FP64: 255 and 168 registers a thread, FP32: 168 and 128 (no spill, a little)
-template <typename R> constexpr int STEPS_BUDGETS[2] = {sizeof(R) == 4 ? 3 : 2, sizeof(R) == 4 ? 4 : 3};
-template <typename R, int NPE, bool ONE, bool PI> int plan_steps_p(dnl_engine *h)
-{
-  const int m = plan_steps_minb<R, NPE, ONE, PI, STEPS_BUDGETS<R>[0]>(h);
-  return m ? m : plan_steps_minb<R, NPE, ONE, PI, STEPS_BUDGETS<R>[1]>(h);
-}
-template <typename R, int NPE, bool ONE> int plan_steps_t(dnl_engine *h)
-{
-  return h->powerIteration ? plan_steps_p<R, NPE, ONE, true>(h) : plan_steps_p<R, NPE, ONE, false>(h);
-}
-
-template <typename R, int NPE, bool ONE, bool PI> int launch_steps_p(dnl_engine *h, const StepsArgs &a)
-{
-  using L = StepsLayout<R, NPE, PI>;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.gridDim = dim3(h->nTiles);
-  cfg.blockDim = dim3(TILE);
-  cfg.dynamicSmemBytes = L::ROW_BYTES + L::STATE_BYTES;
-  cfg.stream = h->stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (h->stepsMinb == STEPS_BUDGETS<R>[0])
-    CK(cudaLaunchKernelEx(&cfg, k_steps<R, NPE, STEPS_BUDGETS<R>[0], ONE, PI>, h->M, a));
-  else
-    CK(cudaLaunchKernelEx(&cfg, k_steps<R, NPE, STEPS_BUDGETS<R>[1], ONE, PI>, h->M, a));
-  return DNL_OK;
-}
-template <typename R, int NPE, bool ONE> int launch_steps_t(dnl_engine *h, const StepsArgs &a)
-{
-  return h->powerIteration ? launch_steps_p<R, NPE, ONE, true>(h, a) : launch_steps_p<R, NPE, ONE, false>(h, a);
-}
-
-// calls f<R, NPE, ONE>(args...) for the engine's precision, element and materials
-#define DNL_STEPS_DISPATCH(f, ...)                                                                                \
-  (h->precision == DNL_PREC_MIXED                                                                                 \
-       ? (h->npe == 8 ? (h->oneMat ? f<float, 8, true>(__VA_ARGS__) : f<float, 8, false>(__VA_ARGS__))            \
-                      : (h->oneMat ? f<float, 4, true>(__VA_ARGS__) : f<float, 4, false>(__VA_ARGS__)))           \
-       : (h->npe == 8 ? (h->oneMat ? f<double, 8, true>(__VA_ARGS__) : f<double, 8, false>(__VA_ARGS__))          \
-                      : (h->oneMat ? f<double, 4, true>(__VA_ARGS__) : f<double, 4, false>(__VA_ARGS__))))
 
 // Whether runs of this engine go through k_steps: a single model whose tiles all fit on the GPU at once at one of the
 // register budgets (FP64: 444 tiles, 7,104 hexahedra; FP32: 592 tiles, 9,472
@@ -735,15 +683,29 @@ template <typename R, int NPE, bool ONE> int launch_steps_t(dnl_engine *h, const
 // (FP64 at 128 registers: 23.3 against 20.4 us on 378 tiles).
 void plan_steps(dnl_engine *h)
 {
-  h->stepsMinb = 0;
+  h->steps = StepsBuild{};
   int coop = 0;
   if (h->nInst != 1 ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device) != cudaSuccess || !coop)
     return;
-  h->stepsMinb = DNL_STEPS_DISPATCH(plan_steps_t, h);
+  for (int k = 0; k < STEPS_BUDGETS && !h->steps.kernel; k++)
+  {
+    const StepsBuild b = h->precision == DNL_PREC_MIXED ? steps_build_of<float>(h, k) : steps_build_of<double>(h, k);
+    if (h->nTiles > b.minb * h->numSMs)
+      continue; // the kernel stays unloaded
+    int perSM = 0;
+    if (cudaFuncSetAttribute(b.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, b.kernel, TILE, b.smem) != cudaSuccess)
+    {
+      cudaGetLastError();
+      perSM = 0;
+    }
+    if (h->nTiles <= perSM * h->numSMs)
+      h->steps = b;
+  }
 }
 
-bool use_steps(const dnl_engine *h) { return h->stepsMinb > 0 && h->mode == DNL_MODE_PLAIN && !h->forced; }
+bool use_steps(const dnl_engine *h) { return h->steps.kernel && h->mode == DNL_MODE_PLAIN && !h->forced; }
 
 // n increments at most (fewer when the model stops) in one launch.
 int launch_steps(dnl_engine *h, int n, bool timed)
@@ -765,9 +727,20 @@ int launch_steps(dnl_engine *h, int n, bool timed)
     a.kin = h->itemsKinetic;
   }
   CK(cudaMemsetAsync(h->stepsBar, 0, 4 * sizeof(unsigned long long), h->stream)); // and the maxima
-  int rc = DNL_STEPS_DISPATCH(launch_steps_t, h, a);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.gridDim = dim3(h->nTiles);
+  cfg.blockDim = dim3(TILE);
+  cfg.dynamicSmemBytes = h->steps.smem;
+  cfg.stream = h->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void *args[] = {&h->M, &a};
+  CK(cudaLaunchKernelExC(&cfg, h->steps.kernel, args));
   h->launches++;
-  return rc;
+  return DNL_OK;
 }
 
 // One increment: the kernels of the graph.
