@@ -179,25 +179,6 @@ __host__ __device__ __forceinline__ double &comp(double4 &v, int c) { return c =
 
 // --------------------------------------------------------------- helpers
 
-// Sum v[] over the NPE lanes of an element group and leave in lane g the DIM
-// values of node g (a butterfly reduce-scatter: NPE/2, NPE/4, ... lanes apart).
-template <typename R, int NPE, int DIM>
-__device__ __forceinline__ void reduce_scatter(unsigned mask, int g, R (&w)[NPE * DIM])
-{
-#pragma unroll
-  for (int half = NPE / 2; half >= 1; half >>= 1)
-  {
-    const bool upper = (g & half) != 0;
-#pragma unroll
-    for (int k = 0; k < half * DIM; k++)
-    {
-      R send = upper ? w[k] : w[k + half * DIM];
-      R keep = upper ? w[k + half * DIM] : w[k];
-      w[k] = keep + __shfl_xor_sync(mask, send, half);
-    }
-  }
-}
-
 template <int NPE> __device__ __forceinline__ float group_sum(unsigned mask, float v)
 {
 #pragma unroll
