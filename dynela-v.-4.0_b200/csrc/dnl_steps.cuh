@@ -108,15 +108,15 @@ __device__ __forceinline__ unsigned long long global_ns()
 
 // I/O of a block whose tile's point state stays in shared memory over the
 // increments of the launch (laid out as in global memory: run ip_slot(c) of
-// TILE values).  When the time step is due the densities go to global memory as
-// well, where the Courant pass reads them.
+// TILE values).  When a Courant time step is due the densities go to global
+// memory as well, where its pass reads them (the power iteration reads none).
 template <typename R, bool ONE> struct ResidentIo
 {
   using R4 = typename V4<R>::type;
   const DevModel &M;
   R *st;
   int t, q, f0, spos;
-  bool due;
+  bool density; // to global memory as well
   __device__ __forceinline__ double4 x(int n) const { return M.x[n]; }
   __device__ __forceinline__ double4 u(int n) const { return M.u[f0][n]; }
   __device__ __forceinline__ const MatDev &mat(int e) const { return M.mat[M.emat[e]]; }
@@ -140,7 +140,7 @@ template <typename R, bool ONE> struct ResidentIo
   __device__ __forceinline__ void put(int c, R v) const
   {
     st[ip_slot(c) * TILE + t] = v;
-    if (c == DNL_IP_DENSITY && due)
+    if (c == DNL_IP_DENSITY && density)
       ipw<R>(M, c, q, v);
   }
   __device__ __forceinline__ void slot(const R4 &v) const { reinterpret_cast<R4 *>(M.slot)[spos] = v; }
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
     if (act)
     {
       SharedTile<R> old{st, te};
-      ResidentIo<R, ONE> io{M, st, te, q, c.f0, spos, due};
+      ResidentIo<R, ONE> io{M, st, te, q, c.f0, spos, !PI && due};
       element_update<R, NPE>(io, &c, M.ctl, q, e, g, base, amask, node, old, rows + te * ROW, rows + (te - g) * ROW);
     }
     if (!(ok = bar.sync()))
@@ -417,15 +417,19 @@ __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
     __syncthreads();
     if (hdue)
     {
-      // a record: the point state where the first block reads it.  The node
-      // vectors stay as they are until the next nodal phase, which waits for
-      // the first block at the barrier before it.
+      // a record: the point state where the first block reads it.  No block
+      // goes on before the first has read the items: what follows changes them
+      // ahead of its next barrier (the imposed-speed nodes' u, v and a by
+      // bc_prep_node, the densities by the element phase when the time step is
+      // due).
       state_out();
       if (!(ok = bar.sync()))
         break;
       if (blockIdx.x == 0 && hslot >= 0)
         history_items<R, TILE>(M, c, A.items, A.off, A.nItems, A.kin,
                                A.hist.rec + (size_t)hslot * (HIST_HEAD + A.nValues) + HIST_HEAD, red);
+      if (!(ok = bar.sync()))
+        break;
     }
     if (stamp)
       ns[2] += global_ns() - t0;
