@@ -9,6 +9,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -71,6 +72,7 @@ struct dnl_engine
   unsigned *stepsBar = nullptr;            // grid barrier
   unsigned long long *stepsPhase = nullptr; // [3] phase times (ns)
   double variantMs[DNL_NUM_VARIANTS] = {0};
+  std::map<const void *, int> resident; // blocks per SM of the kernels asked so far (resident_blocks)
   int *derr = nullptr;      // bulk-copy wait failure flag
   int numSMs = 0;
   bool powerIteration = false;
@@ -313,6 +315,25 @@ void launch_pdl(dnl_engine *h, void (*k)(P...), int grid, int block, size_t smem
   cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// Blocks per SM of a kernel of `threads` threads and `smem` bytes of dynamic
+// shared memory, asked once per engine and kernel: the opt-in to more than
+// 48 KB holds on the device where it was made, and the engines of a process
+// may be on several.
+int resident_blocks(dnl_engine *h, const void *kernel, int threads, size_t smem, int *blocks)
+{
+  auto it = h->resident.find(kernel);
+  if (it == h->resident.end())
+  {
+    int n = 0;
+    if (smem)
+      CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem));
+    it = h->resident.emplace(kernel, std::max(n, 1)).first;
+  }
+  *blocks = it->second;
+  return DNL_OK;
+}
+
 template <typename R, int NPE, bool ONE, int MINB, int PTS = TILE> int launch_plain(dnl_engine *h)
 {
   // work slots: a batch has up to nInst - 1 more slots than tiles (a tile
@@ -327,14 +348,9 @@ template <typename R, int NPE, bool ONE, int MINB, int PTS = TILE> int launch_pl
 template <typename R, int NPE, bool ONE, int MINB> int launch_tma(dnl_engine *h)
 {
   const size_t smem = 2 * (DNL_IP_NREAD * TILE * sizeof(R) + TILE * sizeof(int)) + TILE * ElemShape<NPE>::template pass_row<R> * sizeof(R);
-  static int perSM = -1; // per instantiation
-  if (perSM < 0)
-  {
-    CK(cudaFuncSetAttribute(k_element_tma<R, NPE, MINB, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_element_tma<R, NPE, MINB, ONE>, TILE, smem));
-    if (perSM < 1)
-      perSM = 1;
-  }
+  int perSM = 0, rc = resident_blocks(h, (const void *)k_element_tma<R, NPE, MINB, ONE>, TILE, smem, &perSM);
+  if (rc)
+    return rc;
   const int grid = std::min(h->nTiles, perSM * h->numSMs);
   launch_pdl(h, k_element_tma<R, NPE, MINB, ONE>, grid, TILE, smem, h->M, h->nTiles, h->derr);
   return DNL_OK;
@@ -343,14 +359,9 @@ template <typename R, int NPE, bool ONE, int MINB> int launch_tma(dnl_engine *h)
 template <typename R, int NPE, bool ONE, int MINB> int launch_stage(dnl_engine *h)
 {
   const size_t smem = StageLayout<R, NPE>::BYTES;
-  static int perSM = -1; // per instantiation
-  if (perSM < 0)
-  {
-    CK(cudaFuncSetAttribute(k_element_stage<R, NPE, MINB, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_element_stage<R, NPE, MINB, ONE>, TILE, smem));
-    if (perSM < 1)
-      perSM = 1;
-  }
+  int perSM = 0, rc = resident_blocks(h, (const void *)k_element_stage<R, NPE, MINB, ONE>, TILE, smem, &perSM);
+  if (rc)
+    return rc;
   const int grid = std::min(h->nTiles, perSM * h->numSMs);
   launch_pdl(h, k_element_stage<R, NPE, MINB, ONE>, grid, TILE, smem, h->M, h->nTiles, h->derr);
   return DNL_OK;
@@ -360,14 +371,9 @@ template <typename R, int NPE, bool ONE, bool LOOP, int MINB> int launch_once_t(
 {
   const size_t smem = DNL_IP_NREAD * TILE * sizeof(R) + TILE * ElemShape<NPE>::template pass_row<R> * sizeof(R);
   auto *k = k_element_once<R, NPE, MINB, ONE, LOOP>;
-  static int perSM = -1; // per instantiation
-  if (perSM < 0)
-  {
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, TILE, smem));
-    if (perSM < 1)
-      perSM = 1;
-  }
+  int perSM = 0, rc = resident_blocks(h, (const void *)k, TILE, smem, &perSM);
+  if (rc)
+    return rc;
   const int slots = h->nTiles + h->nInst - 1; // see launch_plain
   launch_pdl(h, k, LOOP ? std::min(slots, ONCE_BLOCKS * perSM * h->numSMs) : slots, TILE, smem, h->M, h->nTiles, h->derr);
   return DNL_OK;
@@ -384,15 +390,9 @@ template <typename R, int NPE, bool ONE, int MINB> int launch_once(dnl_engine *h
 template <int NPE, int MODE> int launch_mode(dnl_engine *h)
 {
   const size_t smem = MODE == MODE_GUESS ? mlp::SMEM_BYTES : 0;
-  static int perSM = -1; // per instantiation
-  if (perSM < 0)
-  {
-    if (smem)
-      CK(cudaFuncSetAttribute(k_element_mode<NPE, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_element_mode<NPE, MODE>, TILE, smem));
-    if (perSM < 1)
-      perSM = 1;
-  }
+  int perSM = 0, rc = resident_blocks(h, (const void *)k_element_mode<NPE, MODE>, TILE, smem, &perSM);
+  if (rc)
+    return rc;
   // the blocks resident on one SM must find their tensor-memory columns free
   if (MODE == MODE_GUESS && perSM * (int)mlp::TMEM_COLS > 512)
     return fail(h, DNL_ERR_CUDA, "guess kernel: %d blocks per SM exceed the tensor memory", perSM);

@@ -391,12 +391,10 @@ int check_err_flag(int *derr, cudaStream_t st)
   return DNL_OK;
 }
 
+// (at each call: the opt-in holds on the current device only)
 bool set_grad_smem()
 {
-  static bool done = false;
-  if (!done)
-    done = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T_BYTES) == cudaSuccess;
-  return done;
+  return cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T_BYTES) == cudaSuccess;
 }
 
 } // namespace dnl_train

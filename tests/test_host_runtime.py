@@ -1,0 +1,82 @@
+"""The engine's host code over a CUDA runtime without a device
+(fake_cudart.cpp: memory is the host's, launches are checked and written down,
+no kernel runs): what one GPU cannot show (several devices) and what a GPU
+should not be made to show (launches that are refused)."""
+import ctypes
+import glob
+import os
+import subprocess
+
+import pytest
+
+import helpers
+from dnlPython import _abi, meshes
+from dnlPython.engine import Engine
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def fake_path(tmp_path_factory):
+    objs = glob.glob(os.path.join(helpers.PKG, "lib", "obj", "*.o"))
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    if not objs or not os.path.exists(os.path.join(cuda, "include", "cuda_runtime_api.h")):
+        pytest.skip("the build's object files or the CUDA headers are not here")
+    out = str(tmp_path_factory.mktemp("fake") / "libdnlgpu_fake.so")
+    # -Bsymbolic: the engine's calls reach the fake also where a CUDA runtime is loaded
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I",
+                    os.path.join(cuda, "include"), "-o", out, os.path.join(HERE, "fake_cudart.cpp")] + objs,
+                   check=True)
+    return out
+
+
+@pytest.fixture
+def fake(fake_path, monkeypatch):
+    monkeypatch.setattr(_abi, "LIB_PATH", fake_path)
+    monkeypatch.setattr(_abi, "_lib", None)
+    lib = _abi.load_library()
+    lib.fake_launch.restype = ctypes.c_char_p
+    lib.fake_used.restype = ctypes.c_size_t
+    lib.fake_reset(2, ctypes.c_size_t(1 << 40))
+    return lib
+
+
+def launches(lib, kernel):
+    """(grid.x, grid.y, threads, dynamic shared memory, device) of the launches of a kernel."""
+    out = []
+    for i in range(lib.fake_launches()):
+        v = (ctypes.c_int * 5)()
+        if kernel in lib.fake_launch(i, v).decode():
+            out.append(tuple(v))
+    return out
+
+
+@pytest.mark.parametrize("precision,variant", [(_abi.PREC_FP64, v) for v in range(_abi.NUM_VARIANTS)]
+                         + [(_abi.PREC_MIXED, v) for v in range(_abi.NUM_VARIANTS)])
+def test_engines_on_two_devices_in_one_process(fake, precision, variant):
+    """Every element-pass variant launches on the second device as on the
+    first: the shared-memory opt-in of a kernel holds per device."""
+    d = meshes.hex_block(3, 3, 3, precision=precision)
+    for device in (0, 1, 0):
+        fake.fake_set_device(device)
+        fake.fake_clear_log()
+        with Engine(d) as e:
+            e.init()
+            e.set_variant(variant)
+            fake.fake_clear_log()
+            e.run(max_incs=2)
+            assert [x[4] for x in launches(fake, "k_element")] == [device] * 2
+
+
+@pytest.mark.parametrize("call", ["dnl_mlp_forward", "dnl_mlp_gradients"])
+def test_network_calls_on_two_devices_in_one_process(fake, call):
+    net, grad = _abi.Mlp(), _abi.Mlp()
+    x = (ctypes.c_float * 5)()
+    y = (ctypes.c_float * 1)()
+    for device in (0, 1):
+        fake.fake_set_device(device)
+        if call == "dnl_mlp_forward":
+            rc = fake.dnl_mlp_forward(ctypes.byref(net), x, 1, y, None)
+        else:
+            rc = fake.dnl_mlp_gradients(ctypes.byref(net), x, y, 1, ctypes.byref(grad), y, None)
+        assert rc == _abi.DNL_OK, fake.dnl_engine_last_error(None)
