@@ -296,23 +296,43 @@ const Variant &variant_of(const dnl_engine *h, int v)
   return h->precision == DNL_PREC_MIXED ? kVariantsF32[v] : kVariantsF64[v];
 }
 
-// A kernel of the increment (element, nodal and Courant passes) launched with
-// programmatic stream serialization (see pdl_wait); in the captured graph
-// this is a programmatic edge.
+// A kernel launched on the engine's stream; an error is this launch's own, and
+// every caller returns it: a graph captured without one of its kernels would
+// go on without it.
 template <typename... P, typename... A>
-void launch_pdl(dnl_engine *h, void (*k)(P...), int grid, int block, size_t smem, A... args)
+int launch_attr(dnl_engine *h, cudaLaunchAttribute *at, void (*k)(P...), int grid, int block, size_t smem, A... args)
 {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = h->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k, args...);
+  cfg.numAttrs = at ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k, args...);
+  if (e == cudaSuccess)
+  {
+    h->launches++;
+    return DNL_OK;
+  }
+  cudaGetLastError();
+  return fail(h, DNL_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+}
+template <typename... P, typename... A>
+int launch(dnl_engine *h, void (*k)(P...), int grid, int block, size_t smem, A... args)
+{
+  return launch_attr(h, nullptr, k, grid, block, smem, args...);
+}
+// A kernel of the increment (element, nodal and Courant passes) launched with
+// programmatic stream serialization (see pdl_wait); in the captured graph
+// this is a programmatic edge.
+template <typename... P, typename... A>
+int launch_pdl(dnl_engine *h, void (*k)(P...), int grid, int block, size_t smem, A... args)
+{
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  return launch_attr(h, &at, k, grid, block, smem, args...);
 }
 
 // Blocks per SM of a kernel of `threads` threads and `smem` bytes of dynamic
@@ -341,8 +361,7 @@ template <typename R, int NPE, bool ONE, int MINB, int PTS = TILE> int launch_pl
   // block, or two blocks per slot
   const int slots = h->nTiles + h->nInst - 1;
   const int grid = PTS >= TILE ? (slots + PTS / TILE - 1) / (PTS / TILE) : 2 * slots;
-  launch_pdl(h, k_element<R, NPE, MINB, PTS, ONE>, grid, PTS, 0, h->M, h->nTiles);
-  return DNL_OK;
+  return launch_pdl(h, k_element<R, NPE, MINB, PTS, ONE>, grid, PTS, 0, h->M, h->nTiles);
 }
 
 template <typename R, int NPE, bool ONE, int MINB> int launch_tma(dnl_engine *h)
@@ -352,8 +371,7 @@ template <typename R, int NPE, bool ONE, int MINB> int launch_tma(dnl_engine *h)
   if (rc)
     return rc;
   const int grid = std::min(h->nTiles, perSM * h->numSMs);
-  launch_pdl(h, k_element_tma<R, NPE, MINB, ONE>, grid, TILE, smem, h->M, h->nTiles, h->derr);
-  return DNL_OK;
+  return launch_pdl(h, k_element_tma<R, NPE, MINB, ONE>, grid, TILE, smem, h->M, h->nTiles, h->derr);
 }
 
 template <typename R, int NPE, bool ONE, int MINB> int launch_stage(dnl_engine *h)
@@ -363,8 +381,7 @@ template <typename R, int NPE, bool ONE, int MINB> int launch_stage(dnl_engine *
   if (rc)
     return rc;
   const int grid = std::min(h->nTiles, perSM * h->numSMs);
-  launch_pdl(h, k_element_stage<R, NPE, MINB, ONE>, grid, TILE, smem, h->M, h->nTiles, h->derr);
-  return DNL_OK;
+  return launch_pdl(h, k_element_stage<R, NPE, MINB, ONE>, grid, TILE, smem, h->M, h->nTiles, h->derr);
 }
 
 template <typename R, int NPE, bool ONE, bool LOOP, int MINB> int launch_once_t(dnl_engine *h)
@@ -375,8 +392,7 @@ template <typename R, int NPE, bool ONE, bool LOOP, int MINB> int launch_once_t(
   if (rc)
     return rc;
   const int slots = h->nTiles + h->nInst - 1; // see launch_plain
-  launch_pdl(h, k, LOOP ? std::min(slots, ONCE_BLOCKS * perSM * h->numSMs) : slots, TILE, smem, h->M, h->nTiles, h->derr);
-  return DNL_OK;
+  return launch_pdl(h, k, LOOP ? std::min(slots, ONCE_BLOCKS * perSM * h->numSMs) : slots, TILE, smem, h->M, h->nTiles, h->derr);
 }
 // (a batch has a material per instance at least)
 template <typename R, int NPE, bool ONE, int MINB> int launch_once(dnl_engine *h)
@@ -397,8 +413,7 @@ template <int NPE, int MODE> int launch_mode(dnl_engine *h)
   if (MODE == MODE_GUESS && perSM * (int)mlp::TMEM_COLS > 512)
     return fail(h, DNL_ERR_CUDA, "guess kernel: %d blocks per SM exceed the tensor memory", perSM);
   const int grid = std::min(h->nTiles, perSM * h->numSMs);
-  k_element_mode<NPE, MODE><<<grid, TILE, smem, h->stream>>>(h->M, h->nTiles, h->derr);
-  return DNL_OK;
+  return launch(h, k_element_mode<NPE, MODE>, grid, TILE, smem, h->M, h->nTiles, h->derr);
 }
 
 template <int NPE> int launch_mode_any(dnl_engine *h)
@@ -454,22 +469,19 @@ template <typename R, int NPE, bool ONE> int launch_variant(dnl_engine *h, int v
 int launch_element_any(dnl_engine *h, int mode)
 {
   const int blocks = (int)(((long)h->nE * h->npe + TILE - 1) / TILE);
-  int rc = DNL_OK;
   if (mode == 1)
   {
     if (h->precision == DNL_PREC_MIXED)
     {
       if (h->npe == 8)
-        k_element_start<float, 8><<<blocks, TILE, 0, h->stream>>>(h->M);
-      else
-        k_element_start<float, 4><<<blocks, TILE, 0, h->stream>>>(h->M);
+        return launch(h, k_element_start<float, 8>, blocks, TILE, 0, h->M);
+      return launch(h, k_element_start<float, 4>, blocks, TILE, 0, h->M);
     }
     else
     {
       if (h->npe == 8)
-        k_element_start<double, 8><<<blocks, TILE, 0, h->stream>>>(h->M);
-      else
-        k_element_start<double, 4><<<blocks, TILE, 0, h->stream>>>(h->M);
+        return launch(h, k_element_start<double, 8>, blocks, TILE, 0, h->M);
+      return launch(h, k_element_start<double, 4>, blocks, TILE, 0, h->M);
     }
   }
   else
@@ -477,28 +489,25 @@ int launch_element_any(dnl_engine *h, int mode)
     if (h->nInst > 1)
     {
       // the running instances of this increment, for the element, nodal and Courant passes
-      k_active_list<<<1, 1024, 0, h->stream>>>(h->M, h->npe);
-      h->launches++;
+      if (int rc = launch(h, k_active_list, 1, 1024, 0, h->M, h->npe))
+        return rc;
     }
     if (h->mode != DNL_MODE_PLAIN)
-      rc = h->npe == 8 ? launch_mode_any<8>(h) : launch_mode_any<4>(h);
+      return h->npe == 8 ? launch_mode_any<8>(h) : launch_mode_any<4>(h);
     else if (h->npe == 4)
     {
       // the axisymmetric models are small: one plain variant
       if (h->precision == DNL_PREC_MIXED)
-        rc = h->oneMat ? launch_plain<float, 4, true, 6>(h) : launch_plain<float, 4, false, 6>(h);
-      else
-        rc = h->oneMat ? launch_plain<double, 4, true, 4>(h) : launch_plain<double, 4, false, 4>(h);
+        return h->oneMat ? launch_plain<float, 4, true, 6>(h) : launch_plain<float, 4, false, 6>(h);
+      return h->oneMat ? launch_plain<double, 4, true, 4>(h) : launch_plain<double, 4, false, 4>(h);
     }
     else if (h->oneMat)
-      rc = h->precision == DNL_PREC_MIXED ? launch_variant<float, 8, true>(h, h->variant)
-                                          : launch_variant<double, 8, true>(h, h->variant);
+      return h->precision == DNL_PREC_MIXED ? launch_variant<float, 8, true>(h, h->variant)
+                                            : launch_variant<double, 8, true>(h, h->variant);
     else
-      rc = h->precision == DNL_PREC_MIXED ? launch_variant<float, 8, false>(h, h->variant)
-                                          : launch_variant<double, 8, false>(h, h->variant);
+      return h->precision == DNL_PREC_MIXED ? launch_variant<float, 8, false>(h, h->variant)
+                                            : launch_variant<double, 8, false>(h, h->variant);
   }
-  h->launches++;
-  return rc;
 }
 
 int launch_nodal(dnl_engine *h)
@@ -511,16 +520,14 @@ int launch_nodal(dnl_engine *h)
     if (h->precision == DNL_PREC_MIXED)
     {
       if (h->dim == 3)
-        k_nodal_batch<float, 3><<<blocks, threads, 0, h->stream>>>(h->M);
-      else
-        k_nodal_batch<float, 2><<<blocks, threads, 0, h->stream>>>(h->M);
+        return launch(h, k_nodal_batch<float, 3>, blocks, threads, 0, h->M);
+      return launch(h, k_nodal_batch<float, 2>, blocks, threads, 0, h->M);
     }
     else
     {
       if (h->dim == 3)
-        k_nodal_batch<double, 3><<<blocks, threads, 0, h->stream>>>(h->M);
-      else
-        k_nodal_batch<double, 2><<<blocks, threads, 0, h->stream>>>(h->M);
+        return launch(h, k_nodal_batch<double, 3>, blocks, threads, 0, h->M);
+      return launch(h, k_nodal_batch<double, 2>, blocks, threads, 0, h->M);
     }
   }
   else
@@ -530,20 +537,16 @@ int launch_nodal(dnl_engine *h)
     if (h->precision == DNL_PREC_MIXED)
     {
       if (h->dim == 3)
-        launch_pdl(h, k_nodal<float, 3>, blocks, threads, 0, h->M);
-      else
-        launch_pdl(h, k_nodal<float, 2>, blocks, threads, 0, h->M);
+        return launch_pdl(h, k_nodal<float, 3>, blocks, threads, 0, h->M);
+      return launch_pdl(h, k_nodal<float, 2>, blocks, threads, 0, h->M);
     }
     else
     {
       if (h->dim == 3)
-        launch_pdl(h, k_nodal<double, 3>, blocks, threads, 0, h->M);
-      else
-        launch_pdl(h, k_nodal<double, 2>, blocks, threads, 0, h->M);
+        return launch_pdl(h, k_nodal<double, 3>, blocks, threads, 0, h->M);
+      return launch_pdl(h, k_nodal<double, 2>, blocks, threads, 0, h->M);
     }
   }
-  h->launches++;
-  return DNL_OK;
 }
 
 int launch_courant(dnl_engine *h, int force)
@@ -552,38 +555,29 @@ int launch_courant(dnl_engine *h, int force)
   if (h->precision == DNL_PREC_MIXED)
   {
     if (h->npe == 8)
-      k_courant<float, 8><<<blocks, threads, 0, h->stream>>>(h->M, force);
-    else
-      k_courant<float, 4><<<blocks, threads, 0, h->stream>>>(h->M, force);
+      return launch(h, k_courant<float, 8>, blocks, threads, 0, h->M, force);
+    return launch(h, k_courant<float, 4>, blocks, threads, 0, h->M, force);
   }
   else
   {
     if (h->npe == 8)
-      k_courant<double, 8><<<blocks, threads, 0, h->stream>>>(h->M, force);
-    else
-      k_courant<double, 4><<<blocks, threads, 0, h->stream>>>(h->M, force);
+      return launch(h, k_courant<double, 8>, blocks, threads, 0, h->M, force);
+    return launch(h, k_courant<double, 4>, blocks, threads, 0, h->M, force);
   }
-  h->launches++;
-  return DNL_OK;
 }
 
 int launch_gather(dnl_engine *h, int what)
 {
   const int threads = 256, blocks = (h->nN + threads - 1) / threads;
   if (h->precision == DNL_PREC_MIXED)
-    k_gather<float><<<blocks, threads, 0, h->stream>>>(h->M, what);
-  else
-    k_gather<double><<<blocks, threads, 0, h->stream>>>(h->M, what);
-  h->launches++;
-  return DNL_OK;
+    return launch(h, k_gather<float>, blocks, threads, 0, h->M, what);
+  return launch(h, k_gather<double>, blocks, threads, 0, h->M, what);
 }
 
 int launch_control(dnl_engine *h, int phase, double t_stop = 0.0, long long max_incs = 0)
 {
   const int threads = 128, blocks = (h->nInst + threads - 1) / threads;
-  k_control<<<blocks, threads, 0, h->stream>>>(h->M, phase, t_stop, max_incs);
-  h->launches++;
-  return DNL_OK;
+  return launch(h, k_control, blocks, threads, 0, h->M, phase, t_stop, max_incs);
 }
 
 int launch_bc_prep(dnl_engine *h)
@@ -591,9 +585,7 @@ int launch_bc_prep(dnl_engine *h)
   if (!h->hasSpeed)
     return DNL_OK;
   const int threads = 128, blocks = (h->nSpeed + threads - 1) / threads;
-  k_bc_prep<<<blocks, threads, 0, h->stream>>>(h->M);
-  h->launches++;
-  return DNL_OK;
+  return launch(h, k_bc_prep, blocks, threads, 0, h->M);
 }
 
 // Power-iteration time step: one cooperative launch (grid barriers inside).
@@ -628,27 +620,23 @@ int launch_step_end(dnl_engine *h)
 {
   if (h->powerIteration)
   {
-    launch_pi(h, 0);
-    return launch_control(h, CTL_FINISH);
+    const int rc = launch_pi(h, 0);
+    return rc ? rc : launch_control(h, CTL_FINISH);
   }
   const int threads = 256;
   const int blocks = std::max(1, std::min((h->nE + threads - 1) / threads, 2 * h->numSMs));
   if (h->precision == DNL_PREC_MIXED)
   {
     if (h->npe == 8)
-      launch_pdl(h, k_courant_finish<float, 8>, blocks, threads, 0, h->M);
-    else
-      launch_pdl(h, k_courant_finish<float, 4>, blocks, threads, 0, h->M);
+      return launch_pdl(h, k_courant_finish<float, 8>, blocks, threads, 0, h->M);
+    return launch_pdl(h, k_courant_finish<float, 4>, blocks, threads, 0, h->M);
   }
   else
   {
     if (h->npe == 8)
-      launch_pdl(h, k_courant_finish<double, 8>, blocks, threads, 0, h->M);
-    else
-      launch_pdl(h, k_courant_finish<double, 4>, blocks, threads, 0, h->M);
+      return launch_pdl(h, k_courant_finish<double, 8>, blocks, threads, 0, h->M);
+    return launch_pdl(h, k_courant_finish<double, 4>, blocks, threads, 0, h->M);
   }
-  h->launches++;
-  return DNL_OK;
 }
 
 // History records of the increment that just ended (single models with
@@ -659,13 +647,10 @@ int launch_history(dnl_engine *h)
     return DNL_OK;
   const int kin = h->itemsKinetic;
   if (h->precision == DNL_PREC_MIXED)
-    launch_pdl(h, k_history_ring<float>, 1, 256, 0, h->M, h->hist, (const int4 *)h->ditems,
-               (const long long *)h->ditemOff, h->nItems, (int)h->nValues, kin);
-  else
-    launch_pdl(h, k_history_ring<double>, 1, 256, 0, h->M, h->hist, (const int4 *)h->ditems,
-               (const long long *)h->ditemOff, h->nItems, (int)h->nValues, kin);
-  h->launches++;
-  return DNL_OK;
+    return launch_pdl(h, k_history_ring<float>, 1, 256, 0, h->M, h->hist, (const int4 *)h->ditems,
+                      (const long long *)h->ditemOff, h->nItems, (int)h->nValues, kin);
+  return launch_pdl(h, k_history_ring<double>, 1, 256, 0, h->M, h->hist, (const int4 *)h->ditems,
+                    (const long long *)h->ditemOff, h->nItems, (int)h->nValues, kin);
 }
 
 // The k_steps builds of the engine's precision, element, materials and time step method.
@@ -746,12 +731,11 @@ int launch_steps(dnl_engine *h, int n, bool timed)
 // One increment: the kernels of the graph.
 int enqueue_step(dnl_engine *h)
 {
-  launch_bc_prep(h);
-  launch_element_any(h, 0);
-  launch_nodal(h);
-  launch_step_end(h);
-  launch_history(h);
-  return DNL_OK;
+  int rc;
+  if ((rc = launch_bc_prep(h)) || (rc = launch_element_any(h, 0)) || (rc = launch_nodal(h)) ||
+      (rc = launch_step_end(h)))
+    return rc;
+  return launch_history(h);
 }
 
 // Increments of one k_steps launch: at 5 to 25 us each a launch lasts 2 to 13 ms.
@@ -814,9 +798,20 @@ int capture_steps(dnl_engine *h, int n, cudaGraph_t *graph, cudaGraphExec_t *exe
 {
   long long before = h->launches;
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  for (int k = 0; k < n; k++)
-    enqueue_step(h);
+  int rc = DNL_OK;
+  for (int k = 0; k < n && !rc; k++)
+    rc = enqueue_step(h);
   cudaError_t e = cudaStreamEndCapture(h->stream, graph);
+  if (rc)
+  {
+    // (a capture that a launch has broken off gives no graph)
+    if (e == cudaSuccess)
+      cudaGraphDestroy(*graph);
+    cudaGetLastError();
+    *graph = nullptr;
+    h->launches = before;
+    return rc;
+  }
   if (e != cudaSuccess)
     return fail(h, DNL_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
   CK(cudaGraphInstantiate(exec, *graph, 0));
@@ -1349,17 +1344,17 @@ int dnl_engine_init(dnl_engine *h)
   if (!h)
     return DNL_ERR_ARG;
   // reference Jacobian, initial point state, element masses -> nodal lumped mass
-  launch_element_any(h, 1);
-  launch_gather(h, 0);
+  int rc;
+  if ((rc = launch_element_any(h, 1)) || (rc = launch_gather(h, 0)))
+    return rc;
   // Solver::computeTimeStep(true) (Explicit.C:156-158)
-  launch_timestep(h, 1);
-  launch_control(h, CTL_INIT_DT);
+  if ((rc = launch_timestep(h, 1)) || (rc = launch_control(h, CTL_INIT_DT)))
+    return rc;
   // first element pass at t_start (Explicit.C:161-181)
-  launch_element_any(h, 0);
-  launch_control(h, CTL_POST_INIT);
+  if ((rc = launch_element_any(h, 0)) || (rc = launch_control(h, CTL_POST_INIT)))
+    return rc;
   CK(cudaGetLastError());
-  int rc = sync_ctl(h);
-  if (rc)
+  if ((rc = sync_ctl(h)))
     return rc;
   rc = check_status(h);
   if (rc)
@@ -1393,7 +1388,8 @@ int dnl_engine_run(dnl_engine *h, double t_pause, int64_t max_incs, int64_t *inc
   for (int i = 0; i < h->nInst; i++)
     CK(cudaMemsetAsync(&h->M.ctl[i].resolves, 0, sizeof(int), h->stream));
   CK(cudaEventRecord(ev0, h->stream));
-  launch_control(h, CTL_LIMITS, t_pause, max_incs);
+  if ((rc = launch_control(h, CTL_LIMITS, t_pause, max_incs)))
+    return rc;
   if (steps)
   {
     // STEPS_CHUNK increments a launch (less when the history ring holds
@@ -1446,19 +1442,24 @@ int dnl_engine_run(dnl_engine *h, double t_pause, int64_t max_incs, int64_t *inc
       for (int s = 0; s < maxChunk; s++)
       {
         cudaEvent_t *es = &e[4 * (size_t)s];
-        launch_bc_prep(h);
+        if ((rc = launch_bc_prep(h)))
+          break;
         CK(cudaEventRecord(es[0], h->stream));
-        launch_element_any(h, 0);
+        if ((rc = launch_element_any(h, 0)))
+          break;
         CK(cudaEventRecord(es[1], h->stream));
-        launch_nodal(h);
+        if ((rc = launch_nodal(h)))
+          break;
         CK(cudaEventRecord(es[2], h->stream));
-        launch_step_end(h);
-        launch_history(h);
+        if ((rc = launch_step_end(h)) || (rc = launch_history(h)))
+          break;
         CK(cudaEventRecord(es[3], h->stream));
         queued++;
         if (max_incs > 0 && steps + queued >= max_incs)
           break;
       }
+      if (rc)
+        break;
       CK(cudaEventSynchronize(e[4 * (size_t)(queued - 1) + 3]));
       for (int s = 0; s < queued; s++)
       {
@@ -1574,9 +1575,8 @@ int dnl_engine_element_pass(dnl_engine *h, double time_step)
     CK(cudaMemcpyAsync(&h->M.ctl[i], &ci, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
   }
   CK(cudaMemcpyAsync(&h->M.ctl[0], &c, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
-  launch_element_any(h, 0);
-  launch_gather(h, 1);
-  launch_control(h, CTL_POST_INIT);
+  if ((rc = launch_element_any(h, 0)) || (rc = launch_gather(h, 1)) || (rc = launch_control(h, CTL_POST_INIT)))
+    return rc;
   CK(cudaGetLastError());
   if ((rc = sync_ctl(h)))
     return rc;
@@ -2285,9 +2285,10 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
-  int best = h->variant;
+  const int before = h->variant;
+  int best = before, rc = DNL_OK;
   double bestMs = 1e30;
-  for (int v = 0; v < kNumVariants; v++)
+  for (int v = 0; v < kNumVariants && !rc; v++)
   {
     if (h->nInst > 1 && (variant_of(h, v).tma == 0 || (v == 0 && h->precision == DNL_PREC_FP64)))
     {
@@ -2299,16 +2300,18 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
     for (auto &p : parts)
       CK(cudaMemcpyAsync(const_cast<void *>(p.src), p.dst, p.bytes, cudaMemcpyDeviceToDevice, h->stream));
     h->variant = v;
-    launch_control(h, CTL_LIMITS, 1e300, steps);
+    rc = launch_control(h, CTL_LIMITS, 1e300, steps);
     double ms = 0.0;
-    for (int k = 0; k < steps; k++)
+    for (int k = 0; k < steps && !rc; k++)
     {
-      launch_bc_prep(h);
+      if ((rc = launch_bc_prep(h)))
+        break;
       CK(cudaEventRecord(e0, h->stream));
-      launch_element_any(h, 0);
+      if ((rc = launch_element_any(h, 0)))
+        break;
       CK(cudaEventRecord(e1, h->stream));
-      launch_nodal(h);
-      launch_step_end(h);
+      if ((rc = launch_nodal(h)) || (rc = launch_step_end(h)))
+        break;
       CK(cudaEventSynchronize(e1));
       float t = 0;
       cudaEventElapsedTime(&t, e0, e1);
@@ -2316,6 +2319,8 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
         ms += t;
     }
     CK(cudaStreamSynchronize(h->stream));
+    if (rc)
+      break;
     CK(cudaGetLastError());
     ms /= (steps > 1 ? steps - 1 : 1);
     h->variantMs[v] = ms;
@@ -2349,7 +2354,9 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
   dnl_pool_free(save, h->stream);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  h->variant = best;
+  h->variant = rc ? before : best;
+  if (rc)
+    return rc;
   h->tuned = true;
   drop_graph(h);
   return check_status(h);

@@ -80,3 +80,44 @@ def test_network_calls_on_two_devices_in_one_process(fake, call):
         else:
             rc = fake.dnl_mlp_gradients(ctypes.byref(net), x, y, 1, ctypes.byref(grad), y, None)
         assert rc == _abi.DNL_OK, fake.dnl_engine_last_error(None)
+
+
+def _refused(call):
+    with pytest.raises(_abi.EngineError) as x:
+        call()
+    assert x.value.code == -2 and "launch failed" in str(x.value)
+
+
+@pytest.mark.parametrize("kernel", ["k_element_once", "k_nodal", "k_courant_finish"])
+@pytest.mark.parametrize("timed", [False, True])
+def test_a_refused_launch_is_an_error_of_every_run(fake, kernel, timed):
+    """A kernel that cannot be launched fails the run that captures it and the
+    next one too (no graph without it is kept); launched again, the run goes on."""
+    with Engine(meshes.hex_block(3, 3, 3)) as e:
+        e.init()
+        e.set_variant(0)
+        e.set_timing(timed)
+        fake.fake_refuse(kernel.encode())
+        for _ in range(2):
+            fake.fake_clear_log()
+            _refused(lambda: e.run(max_incs=20))
+            # (kernel by kernel, those before it have been queued)
+            assert timed or [k for k in ("k_element", "k_nodal", "k_courant") if launches(fake, k)] == []
+        variant = e.variant()[0]
+        _refused(lambda: e.autotune(2))
+        assert e.variant()[0] == variant
+        fake.fake_refuse(b"")
+        fake.fake_clear_log()
+        e.run(max_incs=20)
+        assert len(launches(fake, kernel)) > 0
+
+
+def test_a_refused_launch_is_an_error_of_the_start_and_of_a_pass(fake):
+    with Engine(meshes.hex_block(3, 3, 3)) as e:
+        for kernel in (b"k_element_start", b"k_courant", b"k_control", b"k_element_once"):
+            fake.fake_refuse(kernel)
+            _refused(e.init)
+        fake.fake_refuse(b"")
+        e.init()
+        fake.fake_refuse(b"k_gather")
+        _refused(lambda: e.element_pass(1e-9))
