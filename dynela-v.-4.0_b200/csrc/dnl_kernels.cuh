@@ -64,11 +64,12 @@ __device__ __forceinline__ void pdl_wait()
 
 // A node vector (32 bytes) in one 256-bit load: the element pass gathers two
 // per point, as 16 + 8 bytes each 84.0 us per increment on the 153,600-element
-// bar (mixed), so 83.1.  Not for vectors that the same kernel writes.
+// bar (mixed), so 83.1.  Volatile, so that it stays behind pdl_wait (the compiler
+// sees no memory read in it); not for vectors that the same kernel writes.
 __device__ __forceinline__ double4 ld_vec(const double4 *p)
 {
   double4 v;
-  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
   return v;
 }
 
