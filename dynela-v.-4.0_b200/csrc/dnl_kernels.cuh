@@ -1578,6 +1578,8 @@ __global__ void __launch_bounds__(TILE, MINB) k_element_tma(DevModel M, int nTil
 
 // The old point state of a tile on its way into shared memory: ready() waits
 // for the bulk copy (bounded; false, with the error flag set, when it gave up).
+// The lanes of `mask`, which wait together, get one answer: those that went on
+// alone would wait in the element's shuffles for those that gave up.
 template <typename R> struct ArrivingTile
 {
   const R *buf;
@@ -1585,12 +1587,17 @@ template <typename R> struct ArrivingTile
   uint64_t *bar;
   uint32_t phase;
   int *err;
+  unsigned mask;
   __device__ __forceinline__ bool ready() const
   {
-    if (mbar_wait(bar, phase))
+    const bool here = mbar_wait(bar, phase);
+    if (__all_sync(mask, here))
       return true;
-    atomicExch(err, 1);
-    mbar_wait(bar, phase); // no thread leaves while the copy into the block's memory is in flight
+    if (!here)
+    {
+      atomicExch(err, 1);
+      mbar_wait(bar, phase); // no thread leaves while the copy into the block's memory is in flight
+    }
     return false;
   }
   __device__ __forceinline__ R operator()(int c) const { return buf[ip_slot(c) * TILE + t]; }
@@ -1649,7 +1656,7 @@ __global__ void __launch_bounds__(TILE, MINB) k_element_once(DevModel M, int nTi
     Ctl *C = M.ctl + inst;
     const bool act = e >= C->elem_begin && e < C->elem_end && C->active;
     const unsigned amask = __ballot_sync(0xffffffffu, act);
-    ArrivingTile<R> old{state, t, &bar, phase, err};
+    ArrivingTile<R> old{state, t, &bar, phase, err, act ? amask : ~amask};
     if (act)
     {
       if (LOOP)
