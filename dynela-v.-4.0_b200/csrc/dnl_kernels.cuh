@@ -3491,7 +3491,9 @@ __global__ void __launch_bounds__(256) k_history_ring(DevModel M, HistRing H, co
 // -------------------------------------------------------------- energies
 
 // Sums of fixed order (deterministic), spread over the GPU: the partials of an
-// instance (blockIdx.y) by ENERGY_BLOCKS blocks, then their sum by one warp.
+// instance by ENERGY_BLOCKS blocks (`blocks`; KIN_GROUPS for the kinetic energy
+// alone), then their sum by one warp.  The blocks of all instances follow each
+// other in x, as the other dimensions of a grid end at 65,535.
 // The points go to 256 ENERGY_BLOCKS lanes as the nodes to the lanes of
 // node_kinetic above.  Bound by the latency of its loads; in one block per
 // instance the call on the 153,600-element bar (1.2 million points) took 2,360
@@ -3499,12 +3501,13 @@ __global__ void __launch_bounds__(256) k_history_ring(DevModel M, HistRing H, co
 constexpr int ENERGY_BLOCKS = 256;
 constexpr int ENERGY_PARTS = KIN_GROUPS + 2 * ENERGY_BLOCKS; // doubles per instance: kinetic | internal | inelastic
 template <typename R, int NPE>
-__global__ void __launch_bounds__(256) k_energy_parts(DevModel M, double *part, int speed_field, int points)
+__global__ void __launch_bounds__(256) k_energy_parts(DevModel M, double *part, int speed_field, int points, int blocks)
 {
   __shared__ double sh[3][8];
-  const Ctl &c = M.ctl[blockIdx.y];
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5, b = blockIdx.x;
-  double *out = part + (size_t)blockIdx.y * ENERGY_PARTS;
+  const int inst = blockIdx.x / blocks, b = blockIdx.x % blocks;
+  const Ctl &c = M.ctl[inst];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  double *out = part + (size_t)inst * ENERGY_PARTS;
   double ke = 0.0, ei = 0.0, ep = 0.0;
   if (b < KIN_GROUPS)
   {

@@ -728,6 +728,26 @@ int launch_steps(dnl_engine *h, int n, bool timed)
   return DNL_OK;
 }
 
+template <typename R, int NPE>
+int launch_energies_t(dnl_engine *h, double *dst, int speed_field, int points)
+{
+  const int blocks = points ? ENERGY_BLOCKS : KIN_GROUPS;
+  k_energy_parts<R, NPE><<<(unsigned)blocks * h->nInst, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points,
+                                                                          blocks);
+  k_energy_sum<<<h->nInst, 32, 0, h->stream>>>(h->denergyPart, dst, points);
+  CK(cudaGetLastError());
+  return DNL_OK;
+}
+// Energies of every instance into dst [nInst][3]; points = 0: the kinetic only.
+int launch_energies(dnl_engine *h, double *dst, int speed_field, int points)
+{
+  if (h->precision == DNL_PREC_MIXED)
+    return h->npe == 8 ? launch_energies_t<float, 8>(h, dst, speed_field, points)
+                       : launch_energies_t<float, 4>(h, dst, speed_field, points);
+  return h->npe == 8 ? launch_energies_t<double, 8>(h, dst, speed_field, points)
+                     : launch_energies_t<double, 4>(h, dst, speed_field, points);
+}
+
 // One increment: the kernels of the graph.
 int enqueue_step(dnl_engine *h)
 {
@@ -2028,29 +2048,6 @@ int dnl_engine_set_ips(dnl_engine *h, const double *in)
 
 namespace
 {
-// Energies of every instance into dst [nInst][3]; points = 0: the kinetic only.
-int launch_energies(dnl_engine *h, double *dst, int speed_field, int points)
-{
-  const dim3 grid(points ? ENERGY_BLOCKS : KIN_GROUPS, h->nInst);
-  if (h->precision == DNL_PREC_MIXED)
-  {
-    if (h->npe == 8)
-      k_energy_parts<float, 8><<<grid, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points);
-    else
-      k_energy_parts<float, 4><<<grid, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points);
-  }
-  else
-  {
-    if (h->npe == 8)
-      k_energy_parts<double, 8><<<grid, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points);
-    else
-      k_energy_parts<double, 4><<<grid, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points);
-  }
-  k_energy_sum<<<h->nInst, 32, 0, h->stream>>>(h->denergyPart, dst, points);
-  CK(cudaGetLastError());
-  return DNL_OK;
-}
-
 void free_items(dnl_engine *h)
 {
   dnl_pool_free(h->itemMem, h->stream);

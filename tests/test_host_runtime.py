@@ -121,3 +121,13 @@ def test_a_refused_launch_is_an_error_of_the_start_and_of_a_pass(fake):
         e.init()
         fake.fake_refuse(b"k_gather")
         _refused(lambda: e.element_pass(1e-9))
+
+
+def test_energies_of_more_instances_than_a_grid_has_rows(fake):
+    """65,535 is where the second and third dimension of a grid end."""
+    d = meshes.hex_block(1, 1, 1)
+    with Engine([d] * 65_600) as e:
+        e.init()
+        e.energies(65_599)
+        e.set_items([(_abi.ITEM_KINETIC, f, 65_599) for f in (_abi.NODE_SPEED, _abi.NODE_SPEED_PREV)])
+        e.gather_items()
