@@ -3491,33 +3491,41 @@ __global__ void __launch_bounds__(256) k_history_ring(DevModel M, HistRing H, co
 // -------------------------------------------------------------- energies
 
 // Sums of fixed order (deterministic), spread over the GPU: the partials of an
-// instance by ENERGY_BLOCKS blocks (`blocks`; KIN_GROUPS for the kinetic energy
-// alone), then their sum by one warp.  The blocks of all instances follow each
-// other in x, as the other dimensions of a grid end at 65,535.
-// The points go to 256 ENERGY_BLOCKS lanes as the nodes to the lanes of
-// node_kinetic above.  Bound by the latency of its loads; in one block per
-// instance the call on the 153,600-element bar (1.2 million points) took 2,360
-// us, it takes 41 so.
+// instance by up to ENERGY_BLOCKS blocks (KIN_GROUPS for the kinetic energy),
+// then their sum by one warp.  The points go to 256 ENERGY_BLOCKS lanes as the
+// nodes to the lanes of node_kinetic above; a block whose lanes have no point
+// (no node) of any instance is not launched, its partial is the zero it would
+// write.  Bound by the latency of its loads; in one block per instance the call
+// on the 153,600-element bar (1.2 million points) took 2,360 us, it takes 41 so.
+// The blocks of all instances follow each other in x, as the other dimensions of
+// a grid end at 65,535.
 constexpr int ENERGY_BLOCKS = 256;
-constexpr int ENERGY_PARTS = KIN_GROUPS + 2 * ENERGY_BLOCKS; // doubles per instance: kinetic | internal | inelastic
+struct EnergyArgs
+{
+  int first;                   // instances first, first + 1, ...
+  int speed_field;
+  int kinBlocks, pointBlocks;  // blocks with a node, with a point (0: the kinetic energy only)
+  int blocks;                  // blocks per instance, the larger of both
+  __host__ __device__ int parts() const { return kinBlocks + 2 * pointBlocks; } // doubles per instance: kinetic | internal | inelastic
+};
 template <typename R, int NPE>
-__global__ void __launch_bounds__(256) k_energy_parts(DevModel M, double *part, int speed_field, int points, int blocks)
+__global__ void __launch_bounds__(256) k_energy_parts(DevModel M, double *part, EnergyArgs a)
 {
   __shared__ double sh[3][8];
-  const int inst = blockIdx.x / blocks, b = blockIdx.x % blocks;
-  const Ctl &c = M.ctl[inst];
+  const int k = blockIdx.x / a.blocks, b = blockIdx.x % a.blocks;
+  const Ctl &c = M.ctl[a.first + k];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  double *out = part + (size_t)inst * ENERGY_PARTS;
+  double *out = part + (size_t)k * a.parts();
   double ke = 0.0, ei = 0.0, ep = 0.0;
-  if (b < KIN_GROUPS)
+  if (b < a.kinBlocks)
   {
-    const int fsel = speed_field ? (1 - c.f0) : c.f0;
+    const int fsel = a.speed_field ? (1 - c.f0) : c.f0;
 #pragma unroll 4
     for (int i = c.node_begin + b * 256 + t; i < c.node_end; i += 256 * KIN_GROUPS)
       ke = __dadd_rn(ke, node_kinetic(M, fsel, i));
     ke = warp_sum(ke);
   }
-  if (points)
+  if (b < a.pointBlocks)
   {
     const double wfac = (NPE == 4 && !c.plane) ? 6.28318530717958647692 : 1.0;
 #pragma unroll 4
@@ -3537,24 +3545,26 @@ __global__ void __launch_bounds__(256) k_energy_parts(DevModel M, double *part, 
     sh[2][w] = ep;
   }
   __syncthreads();
-  if (t < 3 && (t > 0 || b < KIN_GROUPS))
-    out[t == 0 ? b : KIN_GROUPS + (t - 1) * ENERGY_BLOCKS + b] = group_total(sh[t]);
+  if (t < 3 && b < (t == 0 ? a.kinBlocks : a.pointBlocks))
+    out[t == 0 ? b : a.kinBlocks + (t - 1) * a.pointBlocks + b] = group_total(sh[t]);
 }
 
-// out: [nInst][3] kinetic, internal, inelastic (points = 0: the kinetic only)
-__global__ void __launch_bounds__(32) k_energy_sum(const double *part, double *out, int points)
+// out: [instances][3] kinetic, internal, inelastic
+__global__ void __launch_bounds__(32) k_energy_sum(const double *part, double *out, EnergyArgs a)
 {
-  const double *p = part + (size_t)blockIdx.x * ENERGY_PARTS;
+  const double *p = part + (size_t)blockIdx.x * a.parts();
   const int lane = threadIdx.x;
-  const double ke = groups_total(p[lane]);
+  const double ke = groups_total(lane < a.kinBlocks ? p[lane] : 0.0);
   double e[2] = {0.0, 0.0};
-  if (points)
-    for (int k = 0; k < 2; k++)
-    {
-      const double *q = p + KIN_GROUPS + k * ENERGY_BLOCKS + lane * (ENERGY_BLOCKS / 32);
-      static_assert(ENERGY_BLOCKS / 32 == 8, "eight partials per lane");
-      e[k] = warp_sum(group_total(q));
-    }
+  for (int k = 0; k < 2 && a.pointBlocks; k++)
+  {
+    double v[8];
+    static_assert(ENERGY_BLOCKS / 32 == 8, "eight partials per lane");
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      v[j] = 8 * lane + j < a.pointBlocks ? p[a.kinBlocks + k * a.pointBlocks + 8 * lane + j] : 0.0;
+    e[k] = warp_sum(group_total(v));
+  }
   if (lane == 0)
   {
     double *o = out + 3 * (size_t)blockIdx.x;

@@ -48,7 +48,8 @@ struct dnl_engine
   const int *dIntOf = nullptr;
   std::vector<Ctl> ctlInit;
   Ctl *hctl = nullptr; // host mirror of the control blocks
-  double *denergy = nullptr, *denergyPart = nullptr;
+  double *denergy = nullptr, *denergyPart = nullptr; // of one call: [3], partials
+  int kinBlocks = 0, pointBlocks = 0;                 // blocks of k_energy_parts for the largest instance
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graphExec = nullptr;
   // graphs of r < graphIncs increments (remExec[r]), for runs of a known
@@ -728,24 +729,22 @@ int launch_steps(dnl_engine *h, int n, bool timed)
   return DNL_OK;
 }
 
-template <typename R, int NPE>
-int launch_energies_t(dnl_engine *h, double *dst, int speed_field, int points)
+template <typename R, int NPE> int launch_energies_t(dnl_engine *h, double *dst, const EnergyArgs &a, int n)
 {
-  const int blocks = points ? ENERGY_BLOCKS : KIN_GROUPS;
-  k_energy_parts<R, NPE><<<(unsigned)blocks * h->nInst, 256, 0, h->stream>>>(h->M, h->denergyPart, speed_field, points,
-                                                                          blocks);
-  k_energy_sum<<<h->nInst, 32, 0, h->stream>>>(h->denergyPart, dst, points);
+  k_energy_parts<R, NPE><<<(unsigned)a.blocks * n, 256, 0, h->stream>>>(h->M, h->denergyPart, a);
+  k_energy_sum<<<n, 32, 0, h->stream>>>(h->denergyPart, dst, a);
   CK(cudaGetLastError());
   return DNL_OK;
 }
-// Energies of every instance into dst [nInst][3]; points = 0: the kinetic only.
-int launch_energies(dnl_engine *h, double *dst, int speed_field, int points)
+// Energies of n instances from `first` on into dst [n][3]; points (one instance
+// only: the room for the partials) false: the kinetic only.
+int launch_energies(dnl_engine *h, double *dst, int speed_field, bool points, int first, int n)
 {
+  const int kin = h->kinBlocks, pts = points ? h->pointBlocks : 0;
+  const EnergyArgs a{first, speed_field, kin, pts, std::max(kin, pts)};
   if (h->precision == DNL_PREC_MIXED)
-    return h->npe == 8 ? launch_energies_t<float, 8>(h, dst, speed_field, points)
-                       : launch_energies_t<float, 4>(h, dst, speed_field, points);
-  return h->npe == 8 ? launch_energies_t<double, 8>(h, dst, speed_field, points)
-                     : launch_energies_t<double, 4>(h, dst, speed_field, points);
+    return h->npe == 8 ? launch_energies_t<float, 8>(h, dst, a, n) : launch_energies_t<float, 4>(h, dst, a, n);
+  return h->npe == 8 ? launch_energies_t<double, 8>(h, dst, a, n) : launch_energies_t<double, 4>(h, dst, a, n);
 }
 
 // One increment: the kernels of the graph.
@@ -1041,6 +1040,17 @@ int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_e
   // ---- device memory of the model: one allocation, carved in 256-byte aligned parts
   const size_t rsz = h->precision == DNL_PREC_MIXED ? 4 : 8;
   const size_t nN = (size_t)h->nN, nI = (size_t)n, nIPpad = (size_t)h->nIPpad, nSp = anySpeed ? nN : 1;
+  // energies: the blocks of k_energy_parts that have a node, a point of the
+  // largest instance; partials of all instances' kinetic energies or one's three
+  int mostNodes = 0, mostElems = 0;
+  for (int i = 0; i < n; i++)
+  {
+    mostNodes = std::max(mostNodes, descs[i]->n_nodes);
+    mostElems = std::max(mostElems, descs[i]->n_elems);
+  }
+  h->kinBlocks = std::min(KIN_GROUPS, (mostNodes + 255) / 256);
+  h->pointBlocks = (int)std::min<long long>(ENERGY_BLOCKS, ((long long)mostElems * h->npe + 255) / 256);
+  const size_t nPart = std::max((size_t)h->kinBlocks * nI, (size_t)h->kinBlocks + 2 * h->pointBlocks);
   // force slots: room for the fixed-stride layout (npe per node) or the CSR one
   const size_t nSlotCap = std::max((size_t)h->nIP, nN * h->npe);
   h->nSlotCap = nSlotCap;
@@ -1060,7 +1070,7 @@ int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_e
                o_mass = reserve(sizeof(double) * nN), o_ctl = reserve(sizeof(Ctl) * nI),
                o_perm = reserve(sizeof(int) * (renum ? nN : 1)),
                // zeroed at creation, from here to o_ip
-               o_energy = reserve(sizeof(double) * (3 + ENERGY_PARTS) * nI), o_err = reserve(sizeof(int)),
+               o_energy = reserve(sizeof(double) * (3 + nPart)), o_err = reserve(sizeof(int)),
                o_stats = reserve(sizeof(unsigned long long) * 5), o_done = reserve(sizeof(unsigned) * 2),
                o_steps = reserve(sizeof(unsigned long long) * 7),
                o_act = reserve(sizeof(int)), o_actlist = reserve(sizeof(int) * nI),
@@ -1117,7 +1127,7 @@ int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_e
   M.ctl = (Ctl *)(A + o_ctl);
   h->dIntOf = renum ? (const int *)(A + o_perm) : nullptr;
   h->denergy = (double *)(A + o_energy);
-  h->denergyPart = h->denergy + 3 * nI;
+  h->denergyPart = h->denergy + 3;
   h->derr = (int *)(A + o_err);
   h->dstats = (unsigned long long *)(A + o_stats);
   M.done_count = (unsigned *)(A + o_done);
@@ -2143,7 +2153,7 @@ int dnl_engine_gather_items(dnl_engine *h, double *out)
     // energies of every instance on both speed fields: field0 then field1
     for (int f = 0; f < 2; f++)
       if ((h->itemsKinetic >> f) & 1)
-        if ((rc = launch_energies(h, h->dkin + 3 * f * h->nInst, f, 0)))
+        if ((rc = launch_energies(h, h->dkin + 3 * f * h->nInst, f, false, 0, h->nInst)))
           return rc;
   }
   const int threads = 128, blocks = (h->nItems + threads - 1) / threads;
@@ -2235,10 +2245,10 @@ int dnl_engine_energies(dnl_engine *h, int32_t i, double out[3])
 {
   if (!h || !out || i < 0 || i >= h->nInst)
     return DNL_ERR_ARG;
-  int rc = launch_energies(h, h->denergy, 0, 1);
+  int rc = launch_energies(h, h->denergy, 0, true, i, 1);
   if (rc)
     return rc;
-  CK(cudaMemcpyAsync(out, h->denergy + 3 * i, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(out, h->denergy, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return DNL_OK;
 }

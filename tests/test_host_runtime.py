@@ -131,3 +131,35 @@ def test_energies_of_more_instances_than_a_grid_has_rows(fake):
         e.energies(65_599)
         e.set_items([(_abi.ITEM_KINETIC, f, 65_599) for f in (_abi.NODE_SPEED, _abi.NODE_SPEED_PREV)])
         e.gather_items()
+
+
+def test_energies_launch_and_keep_what_they_need(fake):
+    """One instance's energies are that instance's work, tiny instances are a
+    block each, and an instance adds no kilobytes of partial sums to a batch."""
+    d = meshes.hex_block(1, 1, 1)
+    used = {}
+    for n in (1000, 2000):
+        before = fake.fake_used(0)
+        with Engine([d] * n) as e:
+            used[n] = fake.fake_used(0) - before
+            e.init()
+            fake.fake_clear_log()
+            e.energies(7)
+            assert [x[0] for x in launches(fake, "k_energy")] == [1, 1]
+            e.set_items([(_abi.ITEM_KINETIC, _abi.NODE_SPEED, k) for k in (0, n - 1)])
+            fake.fake_clear_log()
+            e.gather_items()
+            assert [x[0] for x in launches(fake, "k_energy")] == [n, n]
+    # 8 points and nodes, the control block and the tables: about 6 KB
+    assert (used[2000] - used[1000]) / 1000 < 8192
+    # an ordinary model: a block per 256 points, at most 256
+    with Engine([meshes.hex_block(9, 10, 11), d]) as e:
+        e.init()
+        fake.fake_clear_log()
+        e.energies(1)
+        assert launches(fake, "k_energy_parts")[0][0] == (8 * 990 + 255) // 256
+    with Engine(meshes.hex_block(25, 25, 25)) as e:
+        e.init()
+        fake.fake_clear_log()
+        e.energies()
+        assert launches(fake, "k_energy_parts")[0][0] == 256
