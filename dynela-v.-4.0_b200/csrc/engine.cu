@@ -66,7 +66,7 @@ struct dnl_engine
   int nTiles = 0;
   int variant = 0;          // element-pass kernel variant (see kVariants)
   bool tuned = false;
-  bool forced = false;      // a variant asked for by dnl_engine_set_variant
+  bool forced = false;      // a variant asked for by dnl_engine_set_variant and not chosen again by the autotuner
   // increments in one cooperative launch (dnl_steps.cuh): register budget
   // (blocks per SM), 0 when the model is not run so
   StepsBuild steps;
@@ -2262,8 +2262,13 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
     return DNL_ERR_ARG;
   if (!h->initialized)
     return fail(h, DNL_ERR_ARG, "dnl_engine_init must be called first");
-  if (h->npe != 8 || steps <= 0)
+  if (steps <= 0)
     return DNL_OK;
+  if (h->npe != 8) // one variant
+  {
+    h->forced = false;
+    return DNL_OK;
+  }
   const size_t rsz = h->precision == DNL_PREC_MIXED ? 4 : 8;
   const size_t ipBytes = (size_t)DNL_IP_NCOMP * h->nIPpad * rsz, nb = sizeof(double4) * h->nN;
   struct Saved
@@ -2365,6 +2370,7 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
   if (rc)
     return rc;
   h->tuned = true;
+  h->forced = false; // the engine's own choice again, cooperative increments among it
   drop_graph(h);
   return check_status(h);
 }

@@ -375,7 +375,9 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps);
 #define DNL_NUM_VARIANTS 12
 /* Variant in use and the element-pass time (ms) the autotuner measured for each. */
 int dnl_engine_variant(const dnl_engine *h, int32_t *variant, double ms[DNL_NUM_VARIANTS]);
-/* Force an element-pass variant (0 .. DNL_NUM_VARIANTS-1). */
+/* Force an element-pass variant (0 .. DNL_NUM_VARIANTS-1), kernel by kernel
+ * also for a small model; dnl_engine_autotune leaves the choice to the engine
+ * again. */
 int dnl_engine_set_variant(dnl_engine *h, int32_t variant);
 /* Name of a variant of the precision's list ("stage/4": staged tiles, a
  * register budget of 4 blocks of 128 threads per SM), or NULL. */

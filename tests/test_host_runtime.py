@@ -163,3 +163,21 @@ def test_energies_launch_and_keep_what_they_need(fake):
         fake.fake_clear_log()
         e.energies()
         assert launches(fake, "k_energy_parts")[0][0] == 256
+
+
+@pytest.mark.parametrize("mesh,element", [(lambda: meshes.hex_block(3, 3, 3), "k_element_stage"),
+                                          (lambda: meshes.quad_block(5, 5), "k_element")], ids=["hex", "quad"])
+def test_autotune_after_set_variant_chooses_again(fake, mesh, element):
+    """A variant asked for holds until the autotuner is asked: then a small
+    model runs its increments in cooperative launches again."""
+    with Engine(mesh()) as e:
+        e.init()
+        for asked in (False, True, False):
+            if asked:
+                e.set_variant(6)
+            else:
+                e.autotune(2)
+            for _ in range(2):
+                fake.fake_clear_log()
+                e.run(max_incs=3)
+                assert [bool(launches(fake, k)) for k in ("k_steps", element)] == [not asked, asked]
