@@ -8,7 +8,9 @@
 // predictions 4.75 ms and 2.85.  The pool (cudaMemPool) holds at most
 // DNL_POOL_KEEP bytes that nobody uses, the driver returns what is above at the
 // next synchronisation, and hands blocks from stream to stream in the order of
-// the streams' work.  Thread-safe, as the driver's pools are.  Blocks above
+// the streams' work.  dnl_release_memory (dnl_pool_release) gives back what
+// nobody uses, and so does an allocation that fails, before it tries once more.
+// Thread-safe, as the driver's pools are.  Blocks above
 // DNL_POOL_LARGEST are cudaMalloc's: a pool that has to grow by some 500 MB is
 // slower than cudaMalloc (FP64 bar of 153,600 hexahedra, creation 3.0 against
 // 4 to 6 ms).
@@ -25,3 +27,5 @@ constexpr size_t DNL_POOL_KEEP = 256u << 20, DNL_POOL_LARGEST = 64u << 20;
 cudaError_t dnl_pool_alloc(void **p, size_t bytes, cudaStream_t stream);
 // given back when the work queued on `stream` has completed
 void dnl_pool_free(void *p, cudaStream_t stream);
+// what the current device's pool keeps, given back to the device (waits for it)
+cudaError_t dnl_pool_release(void);

@@ -901,6 +901,15 @@ int dnl_device_count(void)
   return n;
 }
 
+int dnl_release_memory(void)
+{
+  const cudaError_t e = dnl_pool_release();
+  if (e == cudaSuccess)
+    return DNL_OK;
+  cudaGetLastError();
+  return fail(nullptr, DNL_ERR_CUDA, "dnl_release_memory: %s", cudaGetErrorString(e));
+}
+
 const char *dnl_engine_last_error(const dnl_engine *h) { return h ? h->err.c_str() : g_create_err; }
 
 int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_engine **out)

@@ -47,16 +47,40 @@ cudaMemPool_t pool_of_device()
 }
 } // namespace
 
+namespace
+{
+cudaError_t allocate(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream)
+{
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, stream) : cudaMalloc(p, bytes);
+}
+} // namespace
+
+cudaError_t dnl_pool_release(void)
+{
+  cudaMemPool_t pool = pool_of_device();
+  if (!pool)
+    return cudaSuccess;
+  // (blocks are given back in the order of their streams' work)
+  cudaError_t e = cudaDeviceSynchronize();
+  return e == cudaSuccess ? cudaMemPoolTrimTo(pool, 0) : e;
+}
+
 cudaError_t dnl_pool_alloc(void **p, size_t bytes, cudaStream_t stream)
 {
   *p = nullptr;
   if (bytes == 0)
     bytes = 1;
-  cudaMemPool_t pool = bytes <= DNL_POOL_LARGEST ? pool_of_device() : nullptr;
-  if (pool)
-    return cudaMallocFromPoolAsync(p, bytes, pool, stream);
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess)
+  cudaMemPool_t kept = pool_of_device(), pool = bytes <= DNL_POOL_LARGEST ? kept : nullptr;
+  cudaError_t e = allocate(p, bytes, pool, stream);
+  if (e == cudaErrorMemoryAllocation && kept)
+  {
+    // what the pool keeps may be what is missing
+    cudaGetLastError();
+    cudaStreamSynchronize(stream);
+    cudaMemPoolTrimTo(kept, 0);
+    e = allocate(p, bytes, pool, stream);
+  }
+  if (e != cudaSuccess || pool)
     return e;
   try
   {

@@ -297,6 +297,7 @@ def load_library():
         "dnl_engine_batch_create": (ctypes.c_int, [ctypes.POINTER(ctypes.POINTER(ModelDescC)), i32,
                                                    ctypes.POINTER(vp)]),
         "dnl_engine_destroy": (ctypes.c_int, [vp]),
+        "dnl_release_memory": (ctypes.c_int, []),
         "dnl_engine_last_error": (ctypes.c_char_p, [vp]),
         "dnl_engine_init": (ctypes.c_int, [vp]),
         "dnl_engine_run": (ctypes.c_int, [vp, dbl, i64, ctypes.POINTER(i64)]),

@@ -17,6 +17,15 @@ def _pd(a):
     return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
 
 
+def release_memory():
+    """Give the device memory that closed engines and network calls have left
+    with the library (at most 256 MB per GPU) back to the current GPU."""
+    lib = _abi.load_library()
+    rc = lib.dnl_release_memory()
+    if rc != 0:
+        raise _abi.EngineError(rc, lib.dnl_engine_last_error(None).decode())
+
+
 class Engine:
     def __init__(self, descs):
         lib = _abi.load_library()

@@ -185,7 +185,15 @@ int dnl_engine_create(const dnl_model_desc *desc, dnl_engine **out);
  * all of them, each with its own time, time step and material. */
 int dnl_engine_batch_create(const dnl_model_desc *const *descs, int32_t n, dnl_engine **out);
 
+/* Ends an engine.  Up to 256 MB per GPU of the device memory that engines and
+ * network calls give back stay with the library for the next ones (blocks above
+ * 64 MB go back at once): dnl_release_memory returns them. */
 int dnl_engine_destroy(dnl_engine *h);
+
+/* Gives the device memory that the library keeps unused on the current GPU back
+ * to the device; waits for the device.  An engine that finds no room does so by
+ * itself. */
+int dnl_release_memory(void);
 
 /* Text of the last error raised on this handle (or the last create error when h is NULL). */
 const char *dnl_engine_last_error(const dnl_engine *h);

@@ -181,3 +181,42 @@ def test_autotune_after_set_variant_chooses_again(fake, mesh, element):
                 fake.fake_clear_log()
                 e.run(max_incs=3)
                 assert [bool(launches(fake, k)) for k in ("k_steps", element)] == [not asked, asked]
+
+
+def test_memory_of_closed_engines_can_be_given_back(fake):
+    from dnlPython.engine import release_memory
+    release_memory()
+    base = fake.fake_used(0)
+    for _ in range(2):
+        with Engine(meshes.hex_block(8, 8, 8)) as e:
+            e.init()
+            e.ips()
+    assert base < fake.fake_used(0) <= base + (256 << 20)
+    release_memory()
+    assert fake.fake_used(0) == base
+
+
+@pytest.mark.parametrize("n", [8, 36], ids=["pool", "direct"])
+def test_a_model_that_fits_only_with_the_kept_memory(fake, n):
+    """Room that closed engines have left with the library is room for the next
+    engine, whether it takes it from the pool or from the device."""
+    d = meshes.hex_block(n, n, n)
+    fake.dnl_release_memory()
+    base = fake.fake_used(0)
+    with Engine(d):
+        need = fake.fake_used(0) - base
+    fake.dnl_release_memory()
+    small = [Engine(meshes.hex_block(7, 7, 7)) for _ in range(3)]
+    for e in small:
+        e.close()
+    assert fake.fake_used(0) > base
+    fake.fake_set_limit(ctypes.c_size_t(base + need))
+    with Engine(d) as e:
+        e.init()
+    fake.dnl_release_memory()
+    # and a model that does not fit is refused as before, without a trace
+    fake.fake_set_limit(ctypes.c_size_t(base + need - 4096))
+    with pytest.raises(_abi.EngineError, match="out of memory"):
+        Engine(d)
+    fake.dnl_release_memory()
+    assert fake.fake_used(0) == base
