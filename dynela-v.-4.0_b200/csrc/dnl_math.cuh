@@ -361,6 +361,10 @@ template <typename R> struct JCParams
 {
   R A, B, C, n, m, depsp0, Tm, Tref, invTmT, thermal; // invTmT = 1/(Tm-Tref), thermal = tq/(rho0 Cp)
   R twoG, invRho0, K;                                 // 2G, 1/rho0 and the bulk modulus of the return
+  // C and m as eval64 takes them, whose logarithm knows normal numbers only: C
+  // a NaN where a rate over depsp0 is infinite or negative (depsp0 of zero), m so
+  // large that the power is zero where (T - Tref) / (Tm - Tref) is (an infinite Tm)
+  R C64, m64;
 };
 
 // Material constants (Material.h, JohnsonCookLaw.C:132-143) with the derived
@@ -396,11 +400,13 @@ inline MatDev make_mat(const dnl_material &m)
   d.K = m.young / (3.0 * (1.0 - 2.0 * m.poisson));               // Material.h:152-156
   d.heatFrac = m.taylor_quinney / (m.density * m.heat_capacity); // Material.h:165-169
   d.wave2 = m.young * (1.0 - m.poisson) / ((1.0 + m.poisson) * (1.0 - 2.0 * m.poisson)); // Element.C:358
-  d.jc64 = {d.A, d.B, d.C, d.n, d.m, d.depsp0, d.Tm, d.Tref, 1.0 / (d.Tm - d.Tref), d.heatFrac, d.twoG,
-            1.0 / d.rho0, d.K};
+  const double C64 = d.depsp0 >= 1e-280 ? d.C : nan("");
+  const double invTmT = 1.0 / (d.Tm - d.Tref), m64 = invTmT >= 0.0 && invTmT < 1e-300 ? 1e6 * d.m : d.m;
+  d.jc64 = {d.A, d.B, d.C, d.n, d.m, d.depsp0, d.Tm, d.Tref, invTmT, d.heatFrac, d.twoG,
+            1.0 / d.rho0, d.K, C64, m64};
   d.jc32 = {(float)d.A,    (float)d.B,      (float)d.C,    (float)d.n,           (float)d.m,
             (float)d.depsp0, (float)d.Tm,   (float)d.Tref, (float)d.jc64.invTmT, (float)d.heatFrac,
-            (float)d.twoG, (float)(1.0 / d.rho0), (float)d.K};
+            (float)d.twoG, (float)(1.0 / d.rho0), (float)d.K, (float)C64, (float)m64};
   return d;
 }
 
@@ -526,7 +532,7 @@ template <typename R, bool PARAM = false> struct JC
   // saved less: some lane of nearly every warp had to call.)
   __device__ __forceinline__ void eval64(double epsp, double ep, double T, double inv_dt, double &yield, double &hard) const
   {
-    const double n = ld(q->n), m = ld(q->m), dT = T - ld(q->Tref);
+    const double n = ld(q->n), m = ld(q->m64), dT = T - ld(q->Tref);
     const bool rate = ep * inv_dt > ld(q->depsp0), hot = dT > 0.0, warm = hot && T < ld(q->Tm); // warm: neither cold nor molten
     const double re = 1.0 / epsp, rg = 1.0 / ep, rt = 1.0 / dT;
     const TwoDoubles le = log_two(epsp), lr = log_two(ep * inv_dt / ld(q->depsp0)),
@@ -538,13 +544,13 @@ template <typename R, bool PARAM = false> struct JC
       pn = epsp >= 0.0 ? (n > 0.0 ? 0.0 : (n == 0.0 ? 1.0 : __longlong_as_double(0x7ff0000000000000ll)))
                        : __longlong_as_double(0x7ff8000000000000ll);
     const double hard0 = ld(q->A) + ld(q->B) * pn;
-    const double visc0 = rate ? 1.0 + ld(q->C) * lr.hi : 1.0;
+    const double visc0 = rate ? 1.0 + ld(q->C64) * lr.hi : 1.0;
     const double temp0 = warm ? 1.0 - thm : (hot ? 0.0 : 1.0);
     const double hv = hard0 * visc0;
     yield = hv * temp0;
     double h = n * ld(q->B) * (epsp > 0.0 ? pn * re : 0.0) * visc0 * temp0;
     if (rate)
-      h += hard0 * ld(q->C) * temp0 * rg;
+      h += hard0 * ld(q->C64) * temp0 * rg;
     if (warm)
       h -= m * ld(q->thermal) * hv * hv * temp0 * thm * rt;
     hard = h;
@@ -676,6 +682,17 @@ __device__ __forceinline__ int radial_return(const Law &jc, R twoG, R heatFrac, 
   }
   else if (Strial > yield)
   {
+    if constexpr (INLINE)
+    {
+      // eval64's logarithm takes normal numbers (and its select zero): an
+      // infinite plastic strain becomes no number, for which the return does
+      // not converge either, one below the normal numbers the smallest of them
+      const int high = __double2hiint(epsp0);
+      if (high >= 0x7ff00000)
+        epsp0 = __longlong_as_double(0x7ff8000000000000ll);
+      if (high < 0x00100000 && epsp0 > 0.0)
+        epsp0 = 0x1p-1022;
+    }
     R gammaMin = R(0);
     R gammaMax = (Strial - yield) / twoG32;
     gamma = st.gamma;
