@@ -1402,10 +1402,10 @@ template <int NPE> struct TileMap
 
 // Element pass, one thread per Gauss point, state read straight from global memory.
 // One block per work slot (TileMap): a tile of a single model, or a tile of a
-// running instance of a batch (blocks past the slots leave at once).  The
-// same binary serves both, so that a model gives the same bits alone and in a
-// batch; the persistent variants below are the ones that suit the tail of a
-// batch, where few instances still run.
+// running instance of a batch (blocks past the slots leave at once).
+// Quadrilaterals run it alone (kernel by kernel) and in batches; hexahedra
+// alone: the kernels below, whose blocks walk over the slots, suit the tail of
+// a batch, where few instances still run.
 // PTS points per block: TILE (a block per work slot), 2 TILE (two slots per
 // block) or TILE / 2 (two blocks per slot); MINB blocks of PTS threads per SM.
 template <typename R, int NPE, int MINB, int PTS = TILE, bool ONE = false>

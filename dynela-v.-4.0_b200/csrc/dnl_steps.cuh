@@ -267,14 +267,15 @@ __device__ __forceinline__ bool power_iteration(const DevModel &M, const StepsAr
 }
 
 // One tile per block, its point state in shared memory from the first
-// increment of the launch to the last.  Bound by latencies: the return's
-// serial chain (FP64: 7 to 10 of the element phase's 9 to 17 us, a chain of
-// pow, log and divisions per iteration), then the barriers (about 1 us each
-// with the loads after them).  Per increment on the B200, kernel by kernel in
-// graph replays -> here: 800 axisymmetric quads 14.9 -> 12.1 us (FP64) and
-// 11.1 -> 7.4 (mixed), 7,747 plane quads 10.7 -> 7.7 (mixed), 6,048 hexahedra
-// 21.1 -> 20.3 (FP64) and 12.8 -> 9.6 (mixed), 8,960 hexahedra 12.7 -> 11.7
-// (mixed).
+// increment of the launch to the last.  Bound by latencies: in FP64 the element
+// phase, 7.0 (800 quads) to 10.5 us (6,720 hexahedra) of an increment, most of it
+// the return's serial chain (eval64); the nodal phase is 2.5 to 3.6 us, the time
+// step and the end of the increment 0.8 to 1.1 on average, a barrier with the
+// loads after it about 1 in each.  Per increment on the B200, increments 300 to
+// 1,300 of an impact, kernel by kernel in graph replays -> here: 800 axisymmetric
+// quads 14.4 -> 11.2 us (FP64) and 10.7 -> 7.3 (mixed), 7,747 plane quads 15.6 ->
+// 12.7 and 11.0 -> 8.1, 6,048 hexahedra 18.0 -> 15.0 and 12.2 -> 9.6, 6,720 18.6 ->
+// 15.4 (FP64), 8,960 13.1 -> 11.4 (mixed).
 template <typename R, int NPE, int MINB, bool ONE, bool PI>
 __global__ void __launch_bounds__(TILE, MINB) k_steps(DevModel M, StepsArgs A)
 {

@@ -67,8 +67,8 @@ struct dnl_engine
   int variant = 0;          // element-pass kernel variant (see kVariants)
   bool tuned = false;
   bool forced = false;      // a variant asked for by dnl_engine_set_variant and not chosen again by the autotuner
-  // increments in one cooperative launch (dnl_steps.cuh): register budget
-  // (blocks per SM), 0 when the model is not run so
+  // the build that runs increments in one cooperative launch (dnl_steps.cuh);
+  // no kernel where the model is not run so
   StepsBuild steps;
   unsigned *stepsBar = nullptr;            // grid barrier
   unsigned long long *stepsPhase = nullptr; // [3] phase times (ns)
@@ -662,11 +662,13 @@ template <typename R> StepsBuild steps_build_of(const dnl_engine *h, int budget)
   return h->powerIteration ? steps_build<R, 4, true>(h->oneMat, budget) : steps_build<R, 4, false>(h->oneMat, budget);
 }
 
-// Whether runs of this engine go through k_steps: a single model whose tiles all fit on the GPU at once at one of the
-// register budgets (FP64: 444 tiles, 7,104 hexahedra; FP32: 592 tiles, 9,472
-// hexahedra).  At the largest sizes the gain over graph replays is 4 to 8 %,
-// at a few tiles a third; with more blocks per SM the element phase spills
-// (FP64 at 128 registers: 23.3 against 20.4 us on 378 tiles).
+// Whether runs of this engine go through k_steps: a single model whose tiles all
+// fit on the GPU at once at one of the register budgets (of 148 SMs, FP64: 444
+// tiles, 7,104 hexahedra or 14,208 quadrilaterals; FP32: 592 tiles, 9,472 or
+// 18,944).  Near the largest sizes the gain over graph replays is 13 to 17 %, at
+// 25 tiles a quarter to a third (figures at k_steps); with more blocks per SM
+// the element phase spills (FP64 at 128 registers, measured with the law's
+// library calls: 23.3 against 20.4 us on 378 tiles).
 void plan_steps(dnl_engine *h)
 {
   h->steps = StepsBuild{};
@@ -2359,10 +2361,15 @@ int dnl_engine_autotune(dnl_engine *h, int32_t steps)
   // increments later; a model's results should not depend on which of two
   // variants a few per cent apart won a trial of microseconds.  Below 16,000
   // hexahedra the pass of 80 registers (once/6), from there to 180,000 the plain
-  // one of 48, as tuned models of these sizes have run (trials on 39,900 to
-  // 153,600: 3 to 6 % behind once/6), above the fastest, which is once/6 (plate of
-  // 491,520: 206 against 213 for the staged pass and 216 for the plain one).  A
-  // batch is offered variants of one arithmetic only and takes the fastest.
+  // one of 48, because tuned models of these sizes have run so and keep their
+  // results; above the fastest, which is once/6 (plate of 491,520: 206 against
+  // 213 for the staged pass and 216 for the plain one).  What the rule costs, or
+  // gives: us an increment over increments 100 to 600 of a bar, once/6 and
+  // plain/10: 10,150 hexahedra 15.1 and 14.6, 14,025 15.9 and 16.6, 20,916 19.5
+  // and 19.5, 45,760 30.7 and 30.9, 109,340 61.7 and 62.1, 153,600 83.4 and 84.2,
+  // 226,800 124.8 and 126.2; in the first increments, where the trials are, once/6
+  // is 3 to 6 % ahead on 39,900 to 153,600.  A batch is offered variants of one
+  // arithmetic only and takes the fastest.
   if (h->nInst == 1 && h->precision == DNL_PREC_MIXED && h->nE < 180000)
   {
     const int prefer = h->nE < 16000 ? 0 : 10;

@@ -358,9 +358,11 @@ int dnl_engine_timings(const dnl_engine *h, double out[4]);
  * instead of after a replay boundary (1.2 % per increment on the
  * 153,600-element bar from 1 to 8).  A run stops on the same increment
  * either way: the increments past an instance's stop do nothing.  Small single
- * models with the Courant time step (FP64 up to 7,104 hexahedra, mixed up to
- * 9,472) run their increments in cooperative launches instead, unless a
- * variant was set with dnl_engine_set_variant. */
+ * models run their increments in cooperative launches instead, with either time
+ * step method, unless a variant was set with dnl_engine_set_variant or the mode
+ * is not DNL_MODE_PLAIN: those whose tiles of 128 Gauss points fit on the GPU at
+ * once, 3 tiles an SM in FP64 and 4 mixed (on 148 SMs 7,104 and 9,472 hexahedra,
+ * 14,208 and 18,944 quadrilaterals). */
 int dnl_engine_set_graph_increments(dnl_engine *h, int32_t n);
 
 /* Number of kernel launches issued on the device by the last run call. */
@@ -374,14 +376,18 @@ int64_t dnl_engine_launch_count(const dnl_engine *h);
  * state, keeps the fastest for the following runs and restores the state.  On
  * the mixed path a single model of less than 180,000 hexahedra keeps a variant
  * by its size when that is within 10 % of the fastest (once/6, 0, below 16,000,
- * plain/10, 10, above), so that its results do not depend on the trial's timing.
+ * plain/10, 10, above), so that its results hardly depend on the trial's timing.
+ * A small single model goes on in cooperative launches (see
+ * dnl_engine_set_graph_increments); the variant kept is then the one of its
+ * dnl_engine_element_pass.
  * A batch (several instances) is not offered the plain variants (their ms
  * entries are -1): they launch a block per tile of the whole batch at every
  * increment, even when few instances still run.  No counterpart in the
  * reference (its element loop has one implementation). */
 int dnl_engine_autotune(dnl_engine *h, int32_t steps);
 #define DNL_NUM_VARIANTS 12
-/* Variant in use and the element-pass time (ms) the autotuner measured for each. */
+/* Variant of the kernel-by-kernel increments and of dnl_engine_element_pass, and
+ * the element-pass time (ms) the autotuner measured for each. */
 int dnl_engine_variant(const dnl_engine *h, int32_t *variant, double ms[DNL_NUM_VARIANTS]);
 /* Force an element-pass variant (0 .. DNL_NUM_VARIANTS-1), kernel by kernel
  * also for a small model; dnl_engine_autotune leaves the choice to the engine
